@@ -190,7 +190,7 @@ AVBD_DEV unsigned primal_flags(const ContactEval &e)
     unsigned f = 0;
     if (!(e.F.x < 0))
         f |= ad::EF_NCLAMP;
-    if (e.fs > e.bounds && e.fs > 0)
+    if (e.cone)
         f |= ad::EF_CONE;
     return f;
 }
@@ -198,7 +198,7 @@ AVBD_DEV unsigned primal_flags(const ContactEval &e)
 AVBD_DEV unsigned dual_flags(const ContactEval &e, const ContactRec &c, float betaLin)
 {
     unsigned f = primal_flags(e);
-    bool inCone = e.fs <= e.bounds;
+    bool inCone = e.inside;
     if (inCone)
         f |= ad::EF_RAMP_T;
     for (int k = 0; k < 3; ++k)

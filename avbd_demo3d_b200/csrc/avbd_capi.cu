@@ -91,7 +91,10 @@ struct AvbdContext
     int n = 0;
     DArr<float4> pos, quat, initLin, initAng, inertLin, inertAng, vel, angvel, prevVel, massMoment, sizeRad;
     DArr<float4> dqLin, dqAng; // pose - initial pose (linear, qdiff), refreshed wherever the pose is written
+    DArr<float4> massDt2; // massMoment / dt^2
     DArr<float4> initAngInv, inertAngInv; // inverses of the step's initial and inertial orientations
+    // stamped words of the wide iteration kernel (avbd_iterate_flow.cuh): bodies, contacts, joints
+    DArr<float4> bodyFlow, contactFlow, jointFlow;
     DArr<float> friction;
 
     // worlds: static per-world classification, per-step grids (one grid per world)
@@ -173,6 +176,7 @@ struct AvbdContext
     bool hasShapes = false;  // some body is not a box
     bool hasSpheres = false; // rolling friction pass after the velocity update
     int iterBlocks = 0;       // co-resident blocks of the iteration kernel (0: not launchable)
+    int wideBlocks = 0;       // the same for the wide iteration kernel
     DArr<IterSync> iterSync;
     DArr<int> iterDone; // per body: iterations completed in the running iteration launch
     int *hIterError = nullptr; // pinned: barrier expiry of the last iteration kernel
@@ -406,6 +410,11 @@ int reserve_manifolds(AvbdContext *ctx, ManBuf &b, size_t count, size_t used)
     return AVBD_OK;
 }
 
+// Worlds the wide iteration kernel takes (by bodies: the solved ones are counted on the
+// device).
+constexpr int WIDE_MAX_BODIES = 32768;
+bool wide_iterations(const AvbdContext *ctx) { return ctx->wideBlocks > 0 && ctx->n <= WIDE_MAX_BODIES; }
+
 DevBodies dev_bodies(AvbdContext *ctx)
 {
     DevBodies B;
@@ -424,7 +433,9 @@ DevBodies dev_bodies(AvbdContext *ctx)
     B.angvel = ctx->angvel.p;
     B.prevVel = ctx->prevVel.p;
     B.massMoment = ctx->massMoment.p;
+    B.massDt2 = ctx->massDt2.p;
     B.sizeRad = ctx->sizeRad.p;
+    B.flow = wide_iterations(ctx) ? ctx->bodyFlow.p : nullptr;
     B.shape = ctx->hasShapes ? ctx->shape.p : nullptr;
     B.friction = ctx->friction.p;
     return B;
@@ -461,6 +472,9 @@ DevForces dev_forces(AvbdContext *ctx)
     F.adj = ctx->adj.p;
     F.rowStart = ctx->rowStart.p;
     F.rows = ctx->rows.p;
+    const bool wide = wide_iterations(ctx);
+    F.contactFlow = wide ? ctx->contactFlow.p : nullptr;
+    F.jointFlow = wide ? ctx->jointFlow.p : nullptr;
     return F;
 }
 
@@ -1287,6 +1301,15 @@ int init_old_manifolds(AvbdContext *ctx)
     return AVBD_OK;
 }
 
+// The wide iteration kernel's stamped words for `manifolds` manifolds and every joint.
+int flow_reserve(AvbdContext *ctx, size_t manifolds)
+{
+    if (!wide_iterations(ctx))
+        return AVBD_OK;
+    CHECK(reserve(ctx, ctx->contactFlow, 16 * std::max<size_t>(manifolds, 1), false));
+    return reserve(ctx, ctx->jointFlow, 4 * (size_t)std::max(ctx->nJoint, 1), false);
+}
+
 int init_forces_device(AvbdContext *ctx)
 {
     DevBodies B = dev_bodies(ctx);
@@ -1296,6 +1319,7 @@ int init_forces_device(AvbdContext *ctx)
     const int need = std::max(std::max(M, J), 1);
     int *idx = ctx->keepIdx.p;
     int *cnt32 = ctx->keepIdx.p + need;
+    CHECK(flow_reserve(ctx, (size_t)M));
     if (M)
     {
         DevManifolds Md = dev_man(ctx->man[ctx->cur]), Mo = dev_man(ctx->man[ctx->cur ^ 1]);
@@ -1314,7 +1338,7 @@ int init_forces_device(AvbdContext *ctx)
         ctx->launches++;
         // back into the live buffer: no swap
         k_manifold_compact<<<grid_for((long long)M * COMPACT_LANES, 128), 128, 0, ctx->stream>>>(
-            Mo, Md, M, ctx->keep.p, idx, st, false);
+            Mo, Md, M, ctx->keep.p, idx, st, false, dev_forces(ctx).contactFlow);
         LAUNCHED();
     }
     if (J)
@@ -1451,13 +1475,16 @@ int init_forces(AvbdContext *ctx)
         newM = ctx->hScalars[0];
         ManBuf &dst = ctx->man[ctx->cur ^ 1];
         CHECK(reserve_manifolds(ctx, dst, (size_t)std::max<long long>(newM, 1), 0));
-        k_manifold_compact<<<grid_for((long long)M * COMPACT_LANES, 128), 128, 0, ctx->stream>>>(Md, dev_man(dst), M, ctx->keep.p, idx);
+        CHECK(flow_reserve(ctx, (size_t)newM));
+        k_manifold_compact<<<grid_for((long long)M * COMPACT_LANES, 128), 128, 0, ctx->stream>>>(
+            Md, dev_man(dst), M, ctx->keep.p, idx, nullptr, true, dev_forces(ctx).contactFlow);
         LAUNCHED();
         ctx->cur ^= 1;
         ctx->nMan = (int)newM;
     }
     if (J)
     {
+        CHECK(flow_reserve(ctx, 0));
         DevForces F = dev_forces(ctx);
         k_joint_init<<<grid_for(J, 128), 128, 0, ctx->stream>>>(B, F, P, ctx->keep.p, nullptr,
                                                                  &ctx->counters.p->orphans);
@@ -1482,6 +1509,11 @@ int init_forces(AvbdContext *ctx)
             LAUNCHED();
             ctx->jcur = o;
             ctx->nJoint = (int)newJ;
+            if (newJ && wide_iterations(ctx))
+            {
+                k_joint_flow<<<grid_for(newJ, 128), 128, 0, ctx->stream>>>(dev_forces(ctx));
+                LAUNCHED();
+            }
         }
     }
     return AVBD_OK;
@@ -1619,16 +1651,29 @@ int iterate_persistent(AvbdContext *ctx, bool deviceCounts = false, IterTape tap
     const int4 *entries = ctx->solveEntry.p;
     const int *colourStart = ctx->colourStart.p;
     IterSync *sync = ctx->iterSync.p;
-    // per-body completed iterations, from zero in every launch
-    CHECK(reserve(ctx, ctx->iterDone, std::max(ctx->n, 1), false));
-    CU(cudaMemsetAsync(ctx->iterDone.p, 0, sizeof(int) * (size_t)ctx->n, ctx->stream));
-    int *done = ctx->iterDone.p;
     unsigned spinLimit = ctx->waitIteration ? ctx->waitIteration : ITER_SPIN_LIMIT;
     const StepState *st = deviceCounts ? ctx->stepState.p : nullptr;
     const int *orphans = &ctx->counters.p->orphans;
-    void *args[] = {&B, &F, &P, &entries, &colourStart, &nColours, &iterations, &sync, &done, &spinLimit, &st,
-                    &orphans, &tape};
+    if (wide_iterations(ctx))
     {
+        int *error = &sync->error;
+        void *args[] = {&B,     &F,         &P,  &entries, &colourStart, &nColours, &iterations,
+                        &error, &spinLimit, &st, &orphans, &tape};
+        PhaseScope ps(ctx, AVBD_PHASE_PRIMAL);
+        void *kernel = ctx->hasShapes ? (void *)k_iterations_wide<true, false>
+                       : tape.pose    ? (void *)k_iterations_wide<false, true>
+                                      : (void *)k_iterations_wide<false, false>;
+        CU(cudaLaunchCooperativeKernel(kernel, ctx->wideBlocks, WIDE_BLOCK, args, sizeof(WideShared), ctx->stream));
+        LAUNCHED();
+    }
+    else
+    {
+        // per-body completed iterations, from zero in every launch
+        CHECK(reserve(ctx, ctx->iterDone, std::max(ctx->n, 1), false));
+        CU(cudaMemsetAsync(ctx->iterDone.p, 0, sizeof(int) * (size_t)ctx->n, ctx->stream));
+        int *done = ctx->iterDone.p;
+        void *args[] = {&B,    &F,         &P,  &entries, &colourStart, &nColours, &iterations, &sync,
+                        &done, &spinLimit, &st, &orphans, &tape};
         PhaseScope ps(ctx, AVBD_PHASE_PRIMAL);
         // worlds with round bodies run the instance that evaluates their contact offsets
         // (a taped step, boxes only, runs the instance that fills its records)
@@ -2206,11 +2251,13 @@ int upload_bodies(AvbdContext *ctx, const AvbdBodies *b, bool props)
             }
         }
         for (DArr<float4> *a : {&ctx->initLin, &ctx->initAng, &ctx->inertLin, &ctx->inertAng, &ctx->dqLin, &ctx->dqAng,
-                                &ctx->initAngInv, &ctx->inertAngInv})
+                                &ctx->initAngInv, &ctx->inertAngInv, &ctx->massDt2})
         {
             CHECK(reserve(ctx, *a, std::max(n, 1), false));
             CU(cudaMemsetAsync(a->p, 0, sizeof(float4) * std::max(n, 1), ctx->stream));
         }
+        if (wide_iterations(ctx))
+            CHECK(reserve(ctx, ctx->bodyFlow, (size_t)FLOW_STRIDE * std::max(n, 1), false));
         CU(cudaStreamSynchronize(ctx->stream));
     }
     return AVBD_OK;
@@ -2413,6 +2460,17 @@ int avbd_create(AvbdContext **out, int32_t device_ordinal, void *cuda_stream)
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&roundSm, k_iterations<ITER_G, ITER_BLOCK, ITER_SUB, true>,
                                                           ITER_BLOCK, smem) == cudaSuccess)
             ctx->iterBlocks = sms * std::min({iterSm, roundSm, tapeSm});
+        // the wide form, for narrow worlds
+        int wideSm[3] = {0, 0, 0};
+        const void *wide[3] = {(const void *)k_iterations_wide<false, false>, (const void *)k_iterations_wide<true, false>,
+                               (const void *)k_iterations_wide<false, true>};
+        for (int k = 0; k < 3; ++k)
+            if (cudaFuncSetAttribute(wide[k], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WideShared)) !=
+                    cudaSuccess ||
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&wideSm[k], wide[k], WIDE_BLOCK, sizeof(WideShared)) !=
+                    cudaSuccess)
+                wideSm[k] = 0;
+        ctx->wideBlocks = std::min({wideSm[0], wideSm[1], wideSm[2]}) > 0 ? sms : 0;
         cudaGetLastError(); // an unsupported configuration only leaves the per-colour launches
     }
     if (reserve(ctx, ctx->counters, 1, false) || reserve(ctx, ctx->bounds, 8, false) ||
@@ -2447,6 +2505,7 @@ void avbd_destroy(AvbdContext *ctx)
     adjoint_release(ctx);
     for (DArr<float4> *a : {&ctx->pos, &ctx->quat, &ctx->initLin, &ctx->initAng, &ctx->inertLin, &ctx->inertAng,
                             &ctx->dqLin, &ctx->dqAng, &ctx->initAngInv, &ctx->inertAngInv,
+                            &ctx->bodyFlow, &ctx->contactFlow, &ctx->jointFlow, &ctx->massDt2,
                             &ctx->vel, &ctx->angvel, &ctx->prevVel, &ctx->massMoment, &ctx->sizeRad, &ctx->largeLo,
                             &ctx->largeHi, &ctx->largeSphere, &ctx->spring, &ctx->joint[0], &ctx->joint[1]})
         release(*a);

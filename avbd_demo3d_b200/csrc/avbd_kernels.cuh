@@ -18,13 +18,17 @@
 #include "avbd_colour.cuh"
 #include "avbd_math.cuh"
 
+#include <climits>
+
 namespace avbd
 {
 
 constexpr float PENALTY_MIN = 1.0f;
 constexpr float PENALTY_MAX = 10000000000.0f;
 constexpr float COLLISION_MARGIN = 0.01f;
-constexpr float STICK_THRESH = 0.00001f;
+// sqrt(x) < 1e-5 (STICK_THRESH, manifold.cpp), without the root: the smallest float whose
+// correctly rounded root is not below 1e-5 (the root is monotone, so the tests agree).
+constexpr float STICK_THRESH_SQ = 0x1.b7cdfap-34f;
 
 constexpr unsigned ADJ_MANIFOLD = 0u, ADJ_JOINT = 1u, ADJ_SPRING = 2u, ADJ_IGNORE = 3u;
 constexpr unsigned ADJ_INDEX_MASK = (1u << 29) - 1u;
@@ -47,6 +51,10 @@ struct DevBodies
     // qdiff against them in the iterations multiplies by the same inverse
     float4 *initAngInv, *inertAngInv;
     float4 *massMoment, *sizeRad;
+    float4 *massDt2; // massMoment / dt^2, the diagonal of every solve's M/dt^2 (k_warm_start)
+    // the narrow-world iteration kernel's stamped body words (avbd_iterate_flow.cuh); null
+    // where that kernel does not run
+    float4 *flow;
     float *friction;
     float4 *shape; // (type, radius, half length, 0) per body; null when every body is a box
 };
@@ -80,6 +88,9 @@ struct DevForces
     // the constraint rows each body's primal solve stamps, in force order (rows_listed)
     int *rowStart; // n + 1
     int2 *rows;    // (force-list entry, (partner body + 1) << 3 | row of that force)
+    // stamped multiplier words of the narrow-world iteration kernel: 16 float4 per manifold,
+    // 4 per joint (avbd_iterate_flow.cuh)
+    float4 *contactFlow, *jointFlow;
 };
 
 // The reference caps each grid at 2^22 cells (solver.cpp:341-357).
@@ -2070,6 +2081,22 @@ __global__ void k_manifold_init(DevBodies B, DevManifolds M, int count, Params P
         *orphanFlag = 1;
 }
 
+// A joint's stamped words before the first iteration (avbd_iterate_flow.cuh).
+AVBD_DEV void joint_flow_start(float4 *o, const float4 *d)
+{
+    o[0] = f4(xyz(d[4]), __int_as_float(d[4].w != 0.0f ? 1 : 0));
+    for (int k = 1; k < 4; ++k)
+        o[k] = f4(xyz(d[4 + k]), __int_as_float(0));
+}
+
+// The stamped words of joints that a compaction moved.
+__global__ void k_joint_flow(DevForces F)
+{
+    int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j < F.nJoint)
+        joint_flow_start(F.jointFlow + 4 * (size_t)j, F.joint + 8 * (size_t)j);
+}
+
 // Joint::initialize (joint.cpp:35-54)
 __global__ void k_joint_init(DevBodies B, DevForces F, Params P, unsigned char *keep, const StepState *st = nullptr,
                              int *orphanFlag = nullptr)
@@ -2100,6 +2127,8 @@ __global__ void k_joint_init(DevBodies B, DevForces F, Params P, unsigned char *
     d[5] = f4(penAng, 0.0f);
     d[6] = f4(lamLin, 0.0f);
     d[7] = f4(lamAng, 0.0f);
+    if (F.jointFlow)
+        joint_flow_start(F.jointFlow + 4 * (size_t)j, d);
     keep[j] = d4.w != 0.0f ? 0 : 1;
     if (orphanFlag && (ab.x < 0 || B.massMoment[ab.x].x <= 0) && B.massMoment[ab.y].x <= 0)
         *orphanFlag = 1;
@@ -2113,8 +2142,11 @@ constexpr int COMPACT_LANES = 8;
 
 // `flip`: dst becomes the live buffer (the state counts the swap); otherwise dst is the
 // buffer the step started from and stays the live one.
+// `contactFlow`: the kept contacts' stamped words before the first iteration go there too
+// (avbd_iterate_flow.cuh; null: that kernel does not run).
 __global__ void k_manifold_compact(DevManifolds src, DevManifolds dst, int count, const unsigned char *keep,
-                                   const int *newIndex, StepState *st = nullptr, bool flip = true)
+                                   const int *newIndex, StepState *st = nullptr, bool flip = true,
+                                   float4 *contactFlow = nullptr)
 {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int m = (int)(t / COMPACT_LANES), lane = (int)(t % COMPACT_LANES);
@@ -2144,8 +2176,16 @@ __global__ void k_manifold_compact(DevManifolds src, DevManifolds dst, int count
         dst.basis[3 * d + lane] = src.basis[3 * m + lane];
     const float4 *s = src.contact + (size_t)m * 32;
     float4 *o = dst.contact + (size_t)d * 32;
+    float4 *cf = contactFlow ? contactFlow + (size_t)d * 16 : nullptr;
     for (int k = lane; k < 4 * n; k += COMPACT_LANES)
-        o[k] = s[k];
+    {
+        const float4 v = s[k];
+        o[k] = v;
+        if (cf && (k & 3) == 2)
+            cf[2 * (k >> 2)] = make_float4(fabsf(v.y), v.z, v.w, v.x);
+        if (cf && (k & 3) == 3)
+            cf[2 * (k >> 2) + 1] = make_float4(v.x, v.y, v.z, __uint_as_float(__float_as_uint(v.w) >> 31));
+    }
 }
 
 __global__ void k_joint_compact(int count, const unsigned char *keep, const int *newIndex, const int2 *abS,
@@ -2441,6 +2481,20 @@ __global__ void k_step_begin(DevBodies B, const float4 *joint, int nJoint, StepS
 // Body warm start (solver.cpp:1134-1169)
 // ---------------------------------------------------------------------------
 
+// Stamped words of a body in the narrow-world iteration kernel (avbd_iterate_flow.cuh): its
+// orientation, pose difference and position, three floats and a stamp in each 16-byte word.
+// Six words a body (the last unused) keep the words a contact reads in two 32-byte sectors.
+constexpr int FLOW_STRIDE = 6, FLOW_USED = 5;
+AVBD_DEV float4 flow_word(int k, float3 p, float4 q, float3 dl, float3 da, int stamp)
+{
+    const float3 v = k == 0   ? f3(q.x, q.y, q.z)
+                     : k == 1 ? f3(q.w, dl.x, dl.y)
+                     : k == 2 ? f3(dl.z, da.x, da.y)
+                     : k == 3 ? f3(da.z, 0.0f, 0.0f)
+                              : p;
+    return f4(v, __int_as_float(stamp));
+}
+
 __global__ void k_warm_start(DevBodies B, const int *adjStart, Params P, const StepState *st = nullptr)
 {
     int b = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2482,8 +2536,15 @@ __global__ void k_warm_start(DevBodies B, const int *adjStart, Params P, const S
     B.inertAng[b] = inertAng;
     B.initAngInv[b] = qinverse(q0);
     B.inertAngInv[b] = qinverse(inertAng);
-    B.dqLin[b] = f4(sub(pos, pos0), 0.0f);
-    B.dqAng[b] = f4(qdiff(q, q0), 0.0f);
+    const float4 mm4 = B.massMoment[b];
+    const float dt2 = dt * dt;
+    B.massDt2[b] = make_float4(fdiv(mm4.x, dt2), fdiv(mm4.y, dt2), fdiv(mm4.z, dt2), fdiv(mm4.w, dt2));
+    const float3 dl = sub(pos, pos0), da = qdiff(q, q0);
+    B.dqLin[b] = f4(dl, 0.0f);
+    B.dqAng[b] = f4(da, 0.0f);
+    if (B.flow) // stamp 0: before the first iteration
+        for (int k = 0; k < FLOW_USED; ++k)
+            B.flow[(size_t)b * FLOW_STRIDE + k] = flow_word(k, pos, q, dl, da, 0);
 }
 
 // finishStep velocities (solver.cpp:1275-1287); rolling friction is sphere-only
@@ -2707,7 +2768,7 @@ struct ContactEval
 {
     M3 jALin, jBLin, jAAng, jBAng;
     float3 C, F;
-    float fs, bounds;
+    bool inside, cone; // friction force at most its bound; above it (and scaled down)
 };
 
 // F from C with the contact's penalty and multiplier: normal clamp and friction cone
@@ -2717,12 +2778,23 @@ AVBD_DEV void contact_force(ContactEval &e, const ContactRec &c, float friction)
     M3 K = diag(c.pen.x, c.pen.y, c.pen.z);
     float3 F = add(mv(K, e.C), c.lam);
     F.x = rmin(F.x, 0.0f);
-    e.bounds = fabsf(F.x) * friction;
-    e.fs = sqrtf(F.y * F.y + F.z * F.z);
-    if (e.fs > e.bounds && e.fs > 0)
+    const float bounds = fabsf(F.x) * friction, s = F.y * F.y + F.z * F.z;
+    // Inside the cone by more than any rounding of the square, the root and the product, the
+    // root is not needed (100 cycles; squares that could overflow or underflow, and NaN, take
+    // it).
+    e.inside = s <= 0.9999f * (bounds * bounds) && bounds < 1e18f && bounds > 1e-15f;
+    e.cone = false;
+    if (!e.inside)
     {
-        F.y *= e.bounds / e.fs;
-        F.z *= e.bounds / e.fs;
+        const float fs = fsqrt(s);
+        e.inside = fs <= bounds;
+        e.cone = fs > bounds && fs > 0;
+        if (e.cone)
+        {
+            const float scale = fdiv(bounds, fs);
+            F.y *= scale;
+            F.z *= scale;
+        }
     }
     e.F = F;
 }
@@ -2734,11 +2806,11 @@ AVBD_DEV void contact_dual(ContactRec &c, const ContactEval &e, float betaLin)
     c.lam = e.F;
     if (e.F.x < 0)
         c.pen.x = rmin(c.pen.x + betaLin * fabsf(e.C.x), PENALTY_MAX);
-    if (e.fs <= e.bounds)
+    if (e.inside)
     {
         c.pen.y = rmin(c.pen.y + betaLin * fabsf(e.C.y), PENALTY_MAX);
         c.pen.z = rmin(c.pen.z + betaLin * fabsf(e.C.z), PENALTY_MAX);
-        c.stick = sqrtf(e.C.y * e.C.y + e.C.z * e.C.z) < STICK_THRESH;
+        c.stick = e.C.y * e.C.y + e.C.z * e.C.z < STICK_THRESH_SQ;
     }
 }
 
@@ -2816,38 +2888,66 @@ AVBD_DEV M3 gs_ball_socket(int k, float3 v)
     return rows(r0, r1, r2);
 }
 
-// Joint rows (joint.cpp:56-123): part 0 = linear stamp, 1 = diagonalised geometric
-// stiffness added to lhsAng, 2 = angular stamp.
-template <bool COH = false>
-AVBD_DEV unsigned joint_term(const DevBodies &B, const DevForces &F, unsigned j, int part, bool isA, float alpha,
-                             float *t)
+// What joint and spring rows read of a body: its pose.
+struct BodyPose
 {
-    const float4 *d = F.joint + 8 * (size_t)j;
-    int2 ab = F.jointAB[j];
+    float3 p;
+    float4 q;
+};
+
+// A contact's (or a joint's linear part's) contribution to the system of the body with
+// Jacobian rows jLin, jAng.
+AVBD_DEV void contact_stamp(const M3 &jLin, const M3 &jAng, float3 pen, float3 force, float *t)
+{
+    M3 jLinT = trans(jLin), jAngT = trans(jAng);
+    M3 jAngTk = times_diag(jAngT, pen);
+    store_terms(t, mm(times_diag(jLinT, pen), jLin), mm(jAngTk, jAng), mm(jAngTk, jLin), mv(jLinT, force),
+                mv(jAngT, force));
+}
+
+// A joint's linear part (joint.cpp:56-101): this body's Jacobian rows, the force and the two
+// bodies' world arms. d: the joint's record (its constant words 0-3 are read); hasA: body A is
+// a body (else the joint is anchored to the world point rA).
+struct JointLinear
+{
+    M3 jLin, jAng;
+    float3 F, rAW, rBW;
+};
+
+AVBD_DEV JointLinear joint_linear(const float4 *d, bool isA, bool hasA, const BodyPose &A, const BodyPose &Bb,
+                                  float3 pen, float3 lam, float alpha)
+{
     float4 d0 = d[0], d1 = d[1];
-    float3 pB = xyz(ld_state<COH>(B.pos + ab.y));
-    float4 qB = ld_state<COH>(B.quat + ab.y);
+    JointLinear l;
+    float3 rA = xyz(d0), rB = xyz(d1);
+    l.rAW = hasA ? rotate(A.q, rA) : f3(0, 0, 0);
+    l.rBW = rotate(Bb.q, rB);
+    M3 K = diag(pen.x, pen.y, pen.z);
+    float3 C = sub(hasA ? add(A.p, l.rAW) : rA, add(Bb.p, l.rBW));
+    if (isinf(d0.w))
+        C = sub(C, mul(xyz(d[2]), alpha));
+    l.F = add(mv(K, C), lam);
+    const float one = isA ? 1.0f : -1.0f;
+    l.jLin = rows(f3(one, 0, 0), f3(0, one, 0), f3(0, 0, one));
+    l.jAng = isA ? skew(neg(l.rAW)) : skew(l.rBW);
+    return l;
+}
+
+// Joint rows (joint.cpp:56-123): part 0 = linear stamp, 1 = diagonalised geometric
+// stiffness added to lhsAng, 2 = angular stamp. pen, lam: the part's penalty and multiplier
+// (linear for parts 0 and 1, angular for 2).
+AVBD_DEV unsigned joint_rows(const float4 *d, int part, bool isA, bool hasA, const BodyPose &A, const BodyPose &Bb,
+                             float3 pen, float3 lam, float alpha, float *t)
+{
     const M3 I = rows(f3(1, 0, 0), f3(0, 1, 0), f3(0, 0, 1));
     const M3 NI = rows(f3(-1, 0, 0), f3(0, -1, 0), f3(0, 0, -1));
     if (part < 2)
     {
-        float3 rA = xyz(d0), rB = xyz(d1);
-        float3 penLin = xyz(ld_state<COH>(d + 4));
-        float3 rAW = ab.x >= 0 ? rotate(ld_state<COH>(B.quat + ab.x), rA) : f3(0, 0, 0);
-        float3 rBW = rotate(qB, rB);
-        M3 K = diag(penLin.x, penLin.y, penLin.z);
-        float3 C = sub(ab.x >= 0 ? add(xyz(ld_state<COH>(B.pos + ab.x)), rAW) : rA, add(pB, rBW));
-        if (isinf(d0.w))
-            C = sub(C, mul(xyz(d[2]), alpha));
-        float3 Fv = add(mv(K, C), xyz(ld_state<COH>(d + 6)));
+        const JointLinear l = joint_linear(d, isA, hasA, A, Bb, pen, lam, alpha);
+        const float3 rAW = l.rAW, rBW = l.rBW, Fv = l.F;
         if (part == 0)
         {
-            M3 jLin = isA ? I : NI;
-            M3 jAng = isA ? skew(neg(rAW)) : skew(rBW);
-            M3 jLinT = trans(jLin), jAngT = trans(jAng);
-            M3 jAngTk = times_diag(jAngT, penLin);
-            store_terms(t, mm(times_diag(jLinT, penLin), jLin), mm(jAngTk, jAng), mm(jAngTk, jLin), mv(jLinT, Fv),
-                        mv(jAngT, Fv));
+            contact_stamp(l.jLin, l.jAng, pen, Fv, t);
             return KIND_FULL;
         }
         float3 r = isA ? rAW : neg(rBW);
@@ -2862,14 +2962,12 @@ AVBD_DEV unsigned joint_term(const DevBodies &B, const DevForces &F, unsigned j,
         t[E_LA22] = D.r2.z;
         return KIND_LHSANG;
     }
-    float3 penAng = xyz(ld_state<COH>(d + 5));
     float torqueArm = d[3].w;
-    M3 K = diag(penAng.x, penAng.y, penAng.z);
-    float4 qa = ab.x >= 0 ? ld_state<COH>(B.quat + ab.x) : make_float4(0, 0, 0, 1);
-    float3 C = mul(qdiff(qa, qB), torqueArm);
-    if (isinf(d1.w))
+    M3 K = diag(pen.x, pen.y, pen.z);
+    float3 C = mul(qdiff(A.q, Bb.q), torqueArm);
+    if (isinf(d[1].w))
         C = sub(C, mul(xyz(d[3]), alpha));
-    float3 Fv = add(mv(K, C), xyz(ld_state<COH>(d + 7)));
+    float3 Fv = add(mv(K, C), lam);
     M3 jAng = mscale(isA ? I : NI, torqueArm);
     M3 LA = mm(mm(trans(jAng), K), jAng);
     float3 RA = mv(trans(jAng), Fv);
@@ -2885,18 +2983,35 @@ AVBD_DEV unsigned joint_term(const DevBodies &B, const DevForces &F, unsigned j,
     return KIND_ANG;
 }
 
-// Spring row (spring.cpp:27-69)
-template <bool COH = false>
-AVBD_DEV unsigned spring_term(const DevBodies &B, const DevForces &F, unsigned s, bool isA, float *t)
+template <bool COH>
+AVBD_DEV BodyPose load_pose(const DevBodies &B, int b)
 {
-    const float4 *d = F.spring + 2 * (size_t)s;
-    int2 ab = F.springAB[s];
+    BodyPose s;
+    s.p = b >= 0 ? xyz(ld_state<COH>(B.pos + b)) : f3(0, 0, 0);
+    s.q = b >= 0 ? ld_state<COH>(B.quat + b) : make_float4(0, 0, 0, 1);
+    return s;
+}
+
+template <bool COH = false>
+AVBD_DEV unsigned joint_term(const DevBodies &B, const DevForces &F, unsigned j, int part, bool isA, float alpha,
+                             float *t)
+{
+    const float4 *d = F.joint + 8 * (size_t)j;
+    const int2 ab = F.jointAB[j];
+    const BodyPose A = load_pose<COH>(B, ab.x), Bb = load_pose<COH>(B, ab.y);
+    const int k = part < 2 ? 4 : 5;
+    return joint_rows(d, part, isA, ab.x >= 0, A, Bb, xyz(ld_state<COH>(d + k)), xyz(ld_state<COH>(d + k + 2)), alpha,
+                      t);
+}
+
+// Spring row (spring.cpp:27-69); d: the spring's record.
+AVBD_DEV unsigned spring_rows(const float4 *d, bool isA, const BodyPose &A, const BodyPose &Bb, float *t)
+{
     float4 d0 = d[0], d1 = d[1];
     float3 rA = xyz(d0), rB = xyz(d1);
     float rest = d0.w, stiffness = d1.w;
-    float4 qA = ld_state<COH>(B.quat + ab.x), qB = ld_state<COH>(B.quat + ab.y);
-    float3 pA = xform(xyz(ld_state<COH>(B.pos + ab.x)), qA, rA);
-    float3 pB = xform(xyz(ld_state<COH>(B.pos + ab.y)), qB, rB);
+    float3 pA = xform(A.p, A.q, rA);
+    float3 pB = xform(Bb.p, Bb.q, rB);
     float3 dd = sub(pA, pB);
     float dLen = len(dd);
     if (dLen <= 1.0e-6f)
@@ -2907,19 +3022,26 @@ AVBD_DEV unsigned spring_term(const DevBodies &B, const DevForces &F, unsigned s
     float3 jLin, jAng;
     if (isA)
     {
-        float3 rW = rotate(qA, rA);
+        float3 rW = rotate(A.q, rA);
         jLin = n;
         jAng = cross(rW, n);
     }
     else
     {
-        float3 rW = rotate(qB, rB);
+        float3 rW = rotate(Bb.q, rB);
         jLin = neg(n);
         jAng = neg(cross(rW, n));
     }
     store_terms(t, mscale(outer(jLin, jLin), stiffness), mscale(outer(jAng, jAng), stiffness),
                 mscale(outer(jAng, jLin), stiffness), mul(jLin, f), mul(jAng, f));
     return KIND_FULL;
+}
+
+template <bool COH = false>
+AVBD_DEV unsigned spring_term(const DevBodies &B, const DevForces &F, unsigned s, bool isA, float *t)
+{
+    const int2 ab = F.springAB[s];
+    return spring_rows(F.spring + 2 * (size_t)s, isA, load_pose<COH>(B, ab.x), load_pose<COH>(B, ab.y), t);
 }
 
 // Rows a force can stamp during one step, in the order the primal adds them: the contacts
@@ -3053,11 +3175,7 @@ AVBD_DEV unsigned contact_term_self(const DevBodies &B, const DevForces &F, unsi
     // this body's Jacobian rows, formed again from the basis and its arm as
     // eval_contact_arms forms them (fewer values live across the dual update)
     const M3 jLin = isA ? basis : mneg(basis);
-    const M3 jAng = rows(cross(rW, jLin.r0), cross(rW, jLin.r1), cross(rW, jLin.r2));
-    M3 jLinT = trans(jLin), jAngT = trans(jAng);
-    M3 jAngTk = times_diag(jAngT, c.pen);
-    store_terms(t, mm(times_diag(jLinT, c.pen), jLin), mm(jAngTk, jAng), mm(jAngTk, jLin), mv(jLinT, e.F),
-                mv(jAngT, e.F));
+    contact_stamp(jLin, rows(cross(rW, jLin.r0), cross(rW, jLin.r1), cross(rW, jLin.r2)), c.pen, e.F, t);
     return KIND_FULL;
 }
 
@@ -3090,21 +3208,25 @@ AVBD_DEV unsigned listed_row_term(const DevBodies &B, const DevForces &F, int2 r
     }
 }
 
-// Initial system M/dt^2 (solver.cpp:1189-1198) as 27 entries
+// Initial system M/dt^2 (solver.cpp:1189-1198) as 27 entries, for body b at pose p, q:
+// diag(m) / dt2 entry by entry, as the reference divides the whole matrix: the diagonal
+// divided (once per step, massDt2), the off-diagonal zeros' quotient 0 / dt2.
+AVBD_DEV void initial_system_at(const DevBodies &B, int b, float dt, float3 p, float4 q, float *t)
+{
+    const float4 md = B.massDt2[b];
+    const float z = zero_over(dt * dt);
+    M3 lhsLin = rows(f3(md.x, z, z), f3(z, md.x, z), f3(z, z, md.x));
+    M3 lhsAng = rows(f3(md.y, z, z), f3(z, md.z, z), f3(z, z, md.w));
+    M3 lhsCross = diag(0, 0, 0);
+    float3 rhsLin = mv(lhsLin, sub(p, xyz(B.inertLin[b])));
+    float3 rhsAng = mv(lhsAng, qdiff_inv(q, B.inertAngInv[b]));
+    store_terms(t, lhsLin, lhsAng, lhsCross, rhsLin, rhsAng);
+}
+
 template <bool COH = false>
 AVBD_DEV void initial_system(const DevBodies &B, int b, float dt, float *t)
 {
-    float4 mm4 = B.massMoment[b];
-    float dt2 = dt * dt;
-    // diag(m) / dt2 entry by entry, as the reference divides the whole matrix: the
-    // diagonal divided, the off-diagonal zeros' quotient 0 / dt2 formed once
-    const float z = zero_over(dt2), ml = fdiv(mm4.x, dt2);
-    M3 lhsLin = rows(f3(ml, z, z), f3(z, ml, z), f3(z, z, ml));
-    M3 lhsAng = rows(f3(fdiv(mm4.y, dt2), z, z), f3(z, fdiv(mm4.z, dt2), z), f3(z, z, fdiv(mm4.w, dt2)));
-    M3 lhsCross = diag(0, 0, 0);
-    float3 rhsLin = mv(lhsLin, sub(xyz(ld_state<COH>(B.pos + b)), xyz(B.inertLin[b])));
-    float3 rhsAng = mv(lhsAng, qdiff_inv(ld_state<COH>(B.quat + b), B.inertAngInv[b]));
-    store_terms(t, lhsLin, lhsAng, lhsCross, rhsLin, rhsAng);
+    initial_system_at(B, b, dt, xyz(ld_state<COH>(B.pos + b)), ld_state<COH>(B.quat + b), t);
 }
 
 // Shared memory of one primal batch: GPB bodies, G lanes each.
@@ -3416,57 +3538,75 @@ __global__ void k_dual_contacts(DevBodies B, DevManifolds M, int nMan, Params P)
         dual_contact_slot<false, ROUND>(B, M, t, P);
 }
 
-// Joint::updateDual with fracture (joint.cpp:125-182)
+// A joint's multipliers and penalties, and whether it broke.
+struct JointState
+{
+    float3 penLin, penAng, lamLin, lamAng;
+    float broken;
+};
+
+// Joint::updateDual with fracture (joint.cpp:125-182) at the bodies' poses; d: the joint's
+// record (words 0-3 are read).
+AVBD_DEV void joint_dual(const float4 *d, bool hasA, const BodyPose &A, const BodyPose &Bb, const Params &P,
+                         JointState &s)
+{
+    float4 d0 = d[0], d1 = d[1];
+    if (lensq(s.penLin) > 0)
+    {
+        M3 K = diag(s.penLin.x, s.penLin.y, s.penLin.z);
+        float3 pa = hasA ? xform(A.p, A.q, xyz(d0)) : xyz(d0);
+        float3 C = sub(pa, xform(Bb.p, Bb.q, xyz(d1)));
+        if (isinf(d0.w))
+        {
+            C = sub(C, mul(xyz(d[2]), P.alpha));
+            s.lamLin = add(mv(K, C), s.lamLin);
+        }
+        s.penLin = minv(add(s.penLin, mul(absv(C), P.betaLin)), rmin(d0.w, PENALTY_MAX));
+    }
+    if (lensq(s.penAng) > 0)
+    {
+        M3 K = diag(s.penAng.x, s.penAng.y, s.penAng.z);
+        float3 C = mul(qdiff(A.q, Bb.q), d[3].w);
+        if (isinf(d1.w))
+        {
+            C = sub(C, mul(xyz(d[3]), P.alpha));
+            s.lamAng = add(mv(K, C), s.lamAng);
+        }
+        s.penAng = minv(add(s.penAng, mul(absv(C), P.betaAng)), rmin(d1.w, PENALTY_MAX));
+    }
+    float fracture = d[2].w;
+    if (lensq(s.lamAng) > fracture * fracture)
+    {
+        s.penLin = f3(0, 0, 0);
+        s.penAng = f3(0, 0, 0);
+        s.lamLin = f3(0, 0, 0);
+        s.lamAng = f3(0, 0, 0);
+        s.broken = 1.0f;
+    }
+}
+
+AVBD_DEV void store_joint_state(float4 *d, const JointState &s)
+{
+    d[4] = f4(s.penLin, s.broken);
+    d[5] = f4(s.penAng, 0.0f);
+    d[6] = f4(s.lamLin, 0.0f);
+    d[7] = f4(s.lamAng, 0.0f);
+}
+
 template <bool COH>
 AVBD_DEV void dual_joint(const DevBodies &B, const DevForces &F, int j, const Params &P)
 {
     float4 *d = F.joint + 8 * (size_t)j;
-    int2 ab = F.jointAB[j];
-    float4 d0 = d[0], d1 = d[1];
-    float4 d4 = ld_state<COH>(d + 4);
-    float3 penLin = xyz(d4), penAng = xyz(ld_state<COH>(d + 5));
-    float3 lamLin = xyz(ld_state<COH>(d + 6)), lamAng = xyz(ld_state<COH>(d + 7));
-    float brokenFlag = d4.w;
-    float3 pB = xyz(ld_state<COH>(B.pos + ab.y));
-    float4 qB = ld_state<COH>(B.quat + ab.y);
-    if (lensq(penLin) > 0)
-    {
-        M3 K = diag(penLin.x, penLin.y, penLin.z);
-        float3 pa = ab.x >= 0 ? xform(xyz(ld_state<COH>(B.pos + ab.x)), ld_state<COH>(B.quat + ab.x), xyz(d0))
-                              : xyz(d0);
-        float3 C = sub(pa, xform(pB, qB, xyz(d1)));
-        if (isinf(d0.w))
-        {
-            C = sub(C, mul(xyz(d[2]), P.alpha));
-            lamLin = add(mv(K, C), lamLin);
-        }
-        penLin = minv(add(penLin, mul(absv(C), P.betaLin)), rmin(d0.w, PENALTY_MAX));
-    }
-    if (lensq(penAng) > 0)
-    {
-        M3 K = diag(penAng.x, penAng.y, penAng.z);
-        float4 qa = ab.x >= 0 ? ld_state<COH>(B.quat + ab.x) : make_float4(0, 0, 0, 1);
-        float3 C = mul(qdiff(qa, qB), d[3].w);
-        if (isinf(d1.w))
-        {
-            C = sub(C, mul(xyz(d[3]), P.alpha));
-            lamAng = add(mv(K, C), lamAng);
-        }
-        penAng = minv(add(penAng, mul(absv(C), P.betaAng)), rmin(d1.w, PENALTY_MAX));
-    }
-    float fracture = d[2].w;
-    if (lensq(lamAng) > fracture * fracture)
-    {
-        penLin = f3(0, 0, 0);
-        penAng = f3(0, 0, 0);
-        lamLin = f3(0, 0, 0);
-        lamAng = f3(0, 0, 0);
-        brokenFlag = 1.0f;
-    }
-    d[4] = f4(penLin, brokenFlag);
-    d[5] = f4(penAng, 0.0f);
-    d[6] = f4(lamLin, 0.0f);
-    d[7] = f4(lamAng, 0.0f);
+    const int2 ab = F.jointAB[j];
+    const float4 d4 = ld_state<COH>(d + 4);
+    JointState s;
+    s.penLin = xyz(d4);
+    s.broken = d4.w;
+    s.penAng = xyz(ld_state<COH>(d + 5));
+    s.lamLin = xyz(ld_state<COH>(d + 6));
+    s.lamAng = xyz(ld_state<COH>(d + 7));
+    joint_dual(d, ab.x >= 0, load_pose<COH>(B, ab.x), load_pose<COH>(B, ab.y), P, s);
+    store_joint_state(d, s);
 }
 
 __global__ void k_dual_joints(DevBodies B, DevForces F, Params P)
@@ -3480,55 +3620,40 @@ __global__ void k_dual_joints(DevBodies B, DevForces F, Params P)
 // All iterations of a step in one cooperative launch
 // ---------------------------------------------------------------------------
 
-// Bounded grid-wide barrier of the iteration kernel: on expiry the kernel records an
-// error and every block leaves.
+// Contacts between two static bodies have no owning row: nothing moves them, so their
+// update of every iteration runs in turn on the same poses (t = manifold * 8 + slot; lpTape:
+// the taped step's multiplier records, tapeM manifolds to a slice).
+template <bool ROUND>
+AVBD_DEV void orphan_contact_duals(const DevBodies &B, const DevForces &F, const Params &P, long long t,
+                                   int iterations, float4 *lpTape, int tapeM)
+{
+    if ((int)(t & 7) >= F.man.n[t >> 3]) // an empty slot: nothing to load
+        return;
+    int2 ab = F.man.ab[t >> 3];
+    if (B.massMoment[ab.x].x > 0 || B.massMoment[ab.y].x > 0)
+        return;
+    for (int k = 1; k <= iterations; ++k)
+        dual_contact_slot<true, ROUND>(B, F.man, t, P, lpTape ? lpTape + (size_t)k * 16 * tapeM : nullptr);
+}
+
+// Joints without a dynamic body likewise.
+AVBD_DEV void orphan_joint_duals(const DevBodies &B, const DevForces &F, const Params &P, int j, int iterations)
+{
+    int2 ab = F.jointAB[j];
+    if ((ab.x >= 0 && B.massMoment[ab.x].x > 0) || B.massMoment[ab.y].x > 0)
+        return;
+    for (int k = 0; k < iterations; ++k)
+        dual_joint<true>(B, F, j, P);
+}
+
+// Default poll limit of the iteration kernels' waits; `error` is set when one expires.
 constexpr unsigned ITER_SPIN_LIMIT = 1u << 22;
 
 struct IterSync
 {
-    unsigned arrive; // barrier arrivals so far in this launch
     int error;
-    int pad[2];
 };
 
-// Arrivals count up through the launch (the counter starts at zero): barrier k of the
-// launch releases every block once k x gridDim.x blocks have arrived, so the last block's
-// arrival alone opens it.
-AVBD_DEV bool iter_barrier(IterSync *s, unsigned &target, unsigned spinLimit = ITER_SPIN_LIMIT)
-{
-    __shared__ int ok;
-    __syncthreads();
-    target += gridDim.x;
-    if (threadIdx.x == 0)
-    {
-        __threadfence();
-        atomicAdd(&s->arrive, 1u);
-        volatile unsigned *arrive = &s->arrive;
-        unsigned spins = 0;
-        while (*arrive < target && ++spins < spinLimit)
-            if (spins > 256)
-                __nanosleep(32);
-        ok = spins < spinLimit;
-        if (!ok)
-            atomicExch(&s->error, 1);
-        __threadfence();
-    }
-    __syncthreads();
-    return ok && ((volatile int *)&s->error)[0] == 0;
-}
-
-// Solver::iteratePrimalDualCpu (solver.cpp:1177-1271) for every iteration of a step, one
-// block per SM, mutable state read at L2. Per iteration: each colour's bodies in batches of
-// at most GPB per block, spread evenly over the blocks; the block works in independent
-// units of SUB threads. With joints, a grid barrier follows each colour and the joints'
-// dual update each iteration; without, each row waits for its partner's iteration count
-// instead (wait_partner), so blocks and units run ahead of one another. The contacts' dual
-// update of iteration k is done in iteration k + 1 by the row of the body that owns the
-// contact, before that row uses it: the owner is the contact's body with the lower colour
-// (or its only dynamic body), which has not moved yet in iteration k + 1, and neither has
-// the other body, so both poses are those the dual sweep of iteration k reads and every
-// contact's update is the same. After one closing grid barrier, the last iteration's
-// contact updates end the launch.
 // The adjoint's per-iteration record of a taped step (IterFlow's tape fields).
 struct IterTape
 {
@@ -3537,7 +3662,18 @@ struct IterTape
     int n = 0, nMan = 0;
 };
 
-// TAPE: the instance that fills a taped step's records (the others compile without them).
+// Solver::iteratePrimalDualCpu (solver.cpp:1177-1271) for every iteration of a step, one
+// block per SM, mutable state read at L2. Per iteration: each colour's bodies in batches of
+// at most GPB per block, spread evenly over the blocks; the block works in independent
+// units of SUB threads. Each row waits for its partner's iteration count (wait_partner)
+// instead of a grid barrier per colour, so blocks and units run ahead of one another. The
+// dual update of a contact or joint for iteration k is done in iteration k + 1 by the row of
+// the body that owns it, before that row uses it: the owner is the force's body with the
+// lower colour (or its only dynamic body), which has not moved yet in iteration k + 1, and
+// neither has the other body, so both poses are those the dual sweep of iteration k reads
+// and every force's update is the same. The last iteration's updates follow each force's
+// last solve. TAPE: the instance that fills a taped step's records (the others compile
+// without them).
 template <int G, int BLOCK, int SUB, bool ROUND = false, bool TAPE = false>
 __global__ void __launch_bounds__(BLOCK, 1) k_iterations(DevBodies B, DevForces F, Params P, const int4 *entries,
                                                          const int *colourStart, int nColours, int iterations,
@@ -3557,15 +3693,10 @@ __global__ void __launch_bounds__(BLOCK, 1) k_iterations(DevBodies B, DevForces 
     constexpr int GPB = BLOCK / G;
     const long long stride = (long long)gridDim.x * BLOCK;
     const long long tid = (long long)blockIdx.x * BLOCK + threadIdx.x;
-    unsigned target = 0;
-    // rows wait for their partners instead of every colour for the grid; joints' dual
-    // updates are fused into their owners' rows like the contacts'; the last iteration's
-    // dual updates follow each force's last solve, so only forces without a dynamic body
-    // (flagged by the initialisation) need the closing pass
-    const bool barriers = done == nullptr;
-    const bool orphans = barriers || (orphanFlag && *orphanFlag != 0);
+    // only forces without a dynamic body (flagged by the initialisation) need the closing pass
+    const bool orphans = orphanFlag && *orphanFlag != 0;
     IterFlow flow;
-    flow.done = barriers ? nullptr : done;
+    flow.done = done;
     flow.error = &sync->error;
     flow.spinLimit = spinLimit;
     if constexpr (TAPE)
@@ -3578,7 +3709,7 @@ __global__ void __launch_bounds__(BLOCK, 1) k_iterations(DevBodies B, DevForces 
     for (int it = 0; it < iterations; ++it)
     {
         flow.it = it;
-        const bool last = !barriers && it == iterations - 1;
+        const bool last = it == iterations - 1;
         for (int c = 0; c < nColours; ++c)
         {
             // the colour's bodies in equal contiguous batches over every block, as few
@@ -3595,44 +3726,16 @@ __global__ void __launch_bounds__(BLOCK, 1) k_iterations(DevBodies B, DevForces 
                                                          it > 0, sh, flow, last);
                 unit_sync<SUB, BLOCK>(); // the unit's solve threads are done with the shared systems
             }
-            if (barriers && !iter_barrier(sync, target, spinLimit))
-                return;
-        }
-        if (barriers && F.nJoint > 0)
-        {
-            for (long long j = tid; j < F.nJoint; j += stride)
-                dual_joint<true>(B, F, (int)j, P);
-            if (!iter_barrier(sync, target, spinLimit))
-                return;
         }
     }
-    if (iterations <= 0 || !orphans)
+    if (!orphans)
         return;
-    if (!barriers && !iter_barrier(sync, target, spinLimit)) // every body has finished every iteration
-        return;
-    // Contacts between two static bodies have no owning row: nothing moves them, so their
-    // update of every iteration runs here, one after the other on the same poses. (With
-    // barriers, every contact's last update runs here.)
+    // forces between static bodies have no owning row: nothing moves them and no row reads them
     for (long long t = tid; t < 8ll * F.nMan; t += stride)
-    {
-        if ((int)(t & 7) >= F.man.n[t >> 3]) // an empty slot: nothing to load
-            continue;
-        int2 ab = F.man.ab[t >> 3];
-        bool orphan = B.massMoment[ab.x].x <= 0 && B.massMoment[ab.y].x <= 0;
-        if (!orphan && !barriers)
-            continue;
-        for (int r = orphan ? iterations : 1; r > 0; --r) // update r from the end: iteration iterations - r
-            dual_contact_slot<true, ROUND>(B, F.man, t, P, flow.lp_slice(iterations - r + 1));
-    }
+        orphan_contact_duals<ROUND>(B, F, P, t, iterations, flow.lpTape, flow.tapeM);
     // joints without a dynamic body likewise
-    if (!barriers)
-        for (long long j = tid; j < F.nJoint; j += stride)
-        {
-            int2 ab = F.jointAB[j];
-            bool orphan = (ab.x < 0 || B.massMoment[ab.x].x <= 0) && B.massMoment[ab.y].x <= 0;
-            for (int r = orphan ? iterations : 0; r > 0; --r)
-                dual_joint<true>(B, F, (int)j, P);
-        }
+    for (long long j = tid; j < F.nJoint; j += stride)
+        orphan_joint_duals(B, F, P, (int)j, iterations);
 }
 
 // ---------------------------------------------------------------------------
@@ -4007,3 +4110,5 @@ __global__ void __launch_bounds__(COLOUR_FLOW_BLOCK) k_colour_greedy(
 }
 
 } // namespace avbd
+
+#include "avbd_iterate_flow.cuh"

@@ -64,7 +64,14 @@ AVBD_DEV float zero_over(float s)
 AVBD_DEV float3 divs(float3 a, float s) { return f3(fdiv(a.x, s), fdiv(a.y, s), fdiv(a.z, s)); }
 AVBD_DEV float dot(float3 a, float3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 AVBD_DEV float lensq(float3 a) { return dot(a, a); }
-AVBD_DEV float len(float3 a) { return sqrtf(lensq(a)); }
+// sqrt, IEEE round-to-nearest; a zero is returned as it is (its root takes 190 cycles for the
+// whole warp where another takes 100), as fdiv does for zero dividends.
+AVBD_DEV float fsqrt(float x)
+{
+    const float r = sqrtf(opaque(x == 0.0f ? 1.0f : x));
+    return x == 0.0f ? x : r;
+}
+AVBD_DEV float len(float3 a) { return fsqrt(lensq(a)); }
 AVBD_DEV float3 cross(float3 a, float3 b)
 {
     return f3(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
