@@ -984,8 +984,12 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
         CHECK(reserve(ctx, ctx->bpKeysAlt, n, false));
         CHECK(reserve(ctx, ctx->sapVals, n, false));
         CHECK(reserve(ctx, ctx->sapValsAlt, n, false));
-        CHECK(reserve(ctx, ctx->pairCount, n, false));
-        CHECK(reserve(ctx, ctx->pairOffset, n, false));
+        if (n > INT_MAX / SAP_PARTS)
+            return fail(ctx, AVBD_ERR_CAPACITY, "too many bodies (%d) for the sweep-and-prune broadphase", n);
+        const int items = SAP_PARTS * n;
+        const int sweepBlocks = grid_for(32ll * items, SAP_BLOCK);
+        CHECK(reserve(ctx, ctx->pairCount, items, false));
+        CHECK(reserve(ctx, ctx->pairOffset, items, false));
         k_sap_axis<<<W, SAP_TILE, 0, ctx->stream>>>(B, ctx->worldStart.p, ctx->sapAxis.p);
         LAUNCHED();
         k_sap_keys<<<grid_for(n, 256), 256, 0, ctx->stream>>>(B, ctx->bodyWorld.p, ctx->sapAxis.p, ctx->bpKeys.p,
@@ -1002,13 +1006,23 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
         CU(cub::DeviceRadixSort::SortPairs(ctx->cubTemp.p, bytes, dk, dv, n, 0, endBit, ctx->stream));
         ctx->launches++;
         DevForces F = dev_forces(ctx);
-        k_sap_sweep<false><<<grid_for(n, 128), 128, 0, ctx->stream>>>(B, F, ctx->sapAxis.p, dk.Current(),
-                                                                       dv.Current(), n, ctx->pairCount.p, nullptr, 0,
-                                                                       0, cnt);
+        k_sap_sweep<false><<<sweepBlocks, SAP_BLOCK, 0, ctx->stream>>>(B, F, ctx->sapAxis.p, dk.Current(), dv.Current(),
+                                                                       n, ctx->pairCount.p, nullptr, 0, 0, cnt);
         LAUNCHED();
-        CHECK(scan_counts(ctx, ctx->pairCount.p, ctx->pairOffset.p, n, 0));
+        CHECK(scan_counts(ctx, ctx->pairCount.p, ctx->pairOffset.p, items, 0));
         ctx->launches++;
-        k_total<<<1, 1, 0, ctx->stream>>>(ctx->pairOffset.p, ctx->pairCount.p, n, ctx->hScalars);
+        if (deviceCounts)
+        {
+            k_bp_commit<<<1, 1, 0, ctx->stream>>>(ctx->stepState.p, ctx->pairOffset.p, ctx->pairCount.p, items, nullptr,
+                                                  nullptr, 0, nullptr, cnt, (long long)man_capacity(ctx));
+            LAUNCHED();
+            k_sap_sweep<true><<<sweepBlocks, SAP_BLOCK, 0, ctx->stream>>>(
+                B, dev_forces(ctx), ctx->sapAxis.p, dk.Current(), dv.Current(), n, nullptr, ctx->pairOffset.p, 0, 0, cnt,
+                ctx->stepState.p);
+            LAUNCHED();
+            return AVBD_OK;
+        }
+        k_total<<<1, 1, 0, ctx->stream>>>(ctx->pairOffset.p, ctx->pairCount.p, items, ctx->hScalars);
         LAUNCHED();
         CU(cudaStreamSynchronize(ctx->stream));
         CHECK(nonfinite_checked(ctx));
@@ -1017,10 +1031,9 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
         {
             CHECK(reserve_manifolds(ctx, ctx->man[ctx->cur], (size_t)(M0 + P1), (size_t)M0));
             DevForces F2 = dev_forces(ctx);
-            k_sap_sweep<true><<<grid_for(n, 128), 128, 0, ctx->stream>>>(B, F2, ctx->sapAxis.p, dk.Current(),
-                                                                          dv.Current(), n, nullptr,
-                                                                          ctx->pairOffset.p, M0,
-                                                                          (unsigned long long)ctx->nextSeq, cnt);
+            k_sap_sweep<true><<<sweepBlocks, SAP_BLOCK, 0, ctx->stream>>>(
+                B, F2, ctx->sapAxis.p, dk.Current(), dv.Current(), n, nullptr, ctx->pairOffset.p, M0,
+                (unsigned long long)ctx->nextSeq, cnt);
             LAUNCHED();
         }
     }
@@ -1837,12 +1850,13 @@ int push_state(AvbdContext *ctx)
     return AVBD_OK;
 }
 
-// Steps that can keep their counts on the device: the grid broadphase, the single-launch
-// iterations, not while the differentiable step records.
+// Steps that can keep their counts on the device: the grid, LBVH and sweep-and-prune
+// broadphases, the single-launch iterations, not while the differentiable step records.
 bool device_step_ok(const AvbdContext *ctx)
 {
     return ctx->stepMode == AVBD_STEP_DEVICE &&
-           (ctx->params.broadphase == AVBD_BROADPHASE_GRID || ctx->params.broadphase == AVBD_BROADPHASE_LBVH) &&
+           (ctx->params.broadphase == AVBD_BROADPHASE_GRID || ctx->params.broadphase == AVBD_BROADPHASE_LBVH ||
+            ctx->params.broadphase == AVBD_BROADPHASE_SAP) &&
            ctx->iterationMode == AVBD_ITERATIONS_PERSISTENT && ctx->iterBlocks > 0 && !ctx->recording &&
            ctx->params.iterations > 0;
 }

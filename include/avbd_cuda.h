@@ -253,8 +253,8 @@ int avbd_load_batch(AvbdContext *ctx, int32_t num_worlds, const int32_t *world_s
 int avbd_write_bodies(AvbdContext *ctx, const AvbdBodies *bodies);
 
 /* Solver::step() for nsteps steps (solver.cpp:934-937 via stepCpuReference 1036-1041).
- * Asynchronous on the context stream. In AVBD_STEP_DEVICE mode (the default, for the grid
- * broadphase with the single-launch iterations) a step keeps every count it needs on the
+ * Asynchronous on the context stream. In AVBD_STEP_DEVICE mode (the default, for the grid,
+ * LBVH and sweep-and-prune broadphases with the single-launch iterations) a step keeps every count it needs on the
  * device and returns as soon as its launches are issued. A step that cannot run as issued
  * stops on the device before it changes anything, and so does every step issued after
  * it: new pairs that do not fit the manifold buffers, a grid that needs the reference's
