@@ -21,6 +21,8 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -241,6 +243,8 @@ struct AvbdContext
     int stepMode = AVBD_STEP_DEVICE;
     int pendingFast = 0;
     int doneAtConfirm = 0, flipsAtConfirm = 0, curAtConfirm = 0;
+    int stateMan = 0;       // the counts the device state holds while no step is pending
+    long long stateSeq = 0;
     bool stateDirty = true;        // the host changed counts: write them to the device state
     unsigned long long seqBound = 0; // above every sequence number a pending step can create
     long long manifoldSpare = 0;   // manifold room beyond the live count (0: the default policy)
@@ -615,9 +619,8 @@ __global__ void k_state_set(StepState *st, int nMan, unsigned long long nextSeq)
 // After the counting passes of the grid broadphase: the new pairs' total, their place
 // after the live manifolds and their sequence numbers, or a stop when they do not fit or
 // the grid needs the host's cell-count cap.
-__global__ void k_bp_commit(StepState *st, const int *offset, const int *count, int nB, const int *llOffset,
-                            const int *llCount, int nItems, const int *cappedAny, const StepCounters *cnt,
-                            long long capacity)
+__device__ void bp_commit(StepState *st, long long p1, long long p2, const int *cappedAny, const StepCounters *cnt,
+                          long long capacity)
 {
     if (st->abort)
         return;
@@ -626,8 +629,6 @@ __global__ void k_bp_commit(StepState *st, const int *offset, const int *count, 
         st->abort = ABORT_GRID;
         return;
     }
-    long long p1 = nB > 0 ? (long long)offset[nB - 1] + count[nB - 1] : 0;
-    long long p2 = nItems > 0 ? (long long)llOffset[nItems - 1] + llCount[nItems - 1] : 0;
     if ((long long)st->nMan + p1 + p2 > capacity)
     {
         st->abort = ABORT_MANIFOLDS;
@@ -641,23 +642,57 @@ __global__ void k_bp_commit(StepState *st, const int *offset, const int *count, 
     st->created = (int)(p1 + p2);
 }
 
-// End of a device-resident step: an expired iteration wait stops every later step.
-__global__ void k_step_end(StepState *st, const IterSync *sync)
+__global__ void k_bp_commit(StepState *st, const int *offset, const int *count, int nB, const int *llOffset,
+                            const int *llCount, int nItems, const int *cappedAny, const StepCounters *cnt,
+                            long long capacity)
 {
-    if (st->abort)
-        return;
-    if (sync->error)
+    long long p1 = nB > 0 ? (long long)offset[nB - 1] + count[nB - 1] : 0;
+    long long p2 = nItems > 0 ? (long long)llOffset[nItems - 1] + llCount[nItems - 1] : 0;
+    bp_commit(st, p1, p2, cappedAny, cnt, capacity);
+}
+
+// The same with the scans of both counts in the launch (lists up to SCAN_SMALL).
+__global__ void __launch_bounds__(SCAN_BLOCK) k_bp_scan_commit(StepState *st, int *offset, const int *count, int nB,
+                                                               int *llOffset, const int *llCount, int nItems,
+                                                               const int *cappedAny, const StepCounters *cnt,
+                                                               long long capacity)
+{
+    const long long p1 = block_scan(nB, [&](int i) { return count[i]; }, [&](int i, int at) { offset[i] = at; });
+    const long long p2 =
+        block_scan(nItems, [&](int i) { return llCount[i]; }, [&](int i, int at) { llOffset[i] = at; });
+    if (threadIdx.x == 0)
+        bp_commit(st, p1, p2, cappedAny, cnt, capacity);
+}
+
+// End of a device-resident step: an expired iteration wait stops every later step. The state,
+// the counters and the colour ranges go to page-locked host memory (written in place: three
+// copies fewer in the stream).
+__global__ void k_step_end(StepState *st, const IterSync *sync, const StepCounters *cnt, const int *colourStart,
+                           StepState *hostState, StepCounters *hostCounters, int *hostStarts)
+{
+    if (threadIdx.x == 0)
     {
-        st->error = STEP_ERR_ITERATION;
-        st->abort = ABORT_ERROR;
-        return;
+        if (!st->abort)
+        {
+            if (sync->error)
+            {
+                st->error = STEP_ERR_ITERATION;
+                st->abort = ABORT_ERROR;
+            }
+            else
+                st->stepsDone++;
+        }
+        *hostState = *st;
+        *hostCounters = *cnt;
     }
-    st->stepsDone++;
+    for (int k = threadIdx.x; k < 257; k += blockDim.x)
+        hostStarts[k] = colourStart[k];
 }
 
 // Per-body force lists (CSR) sorted newest first.
 template <class Key>
-int build_rows(AvbdContext *ctx, const Key *sortedKeys, int total, size_t manifolds, const StepState *st = nullptr);
+int build_rows(AvbdContext *ctx, const Key *sortedKeys, const unsigned *sortedVals, int total, size_t manifolds,
+               const StepState *st = nullptr);
 
 // Bits needed to write v (0 for v = 0).
 int bit_width(unsigned long long v) { return v ? 64 - __builtin_clzll(v) : 0; }
@@ -682,7 +717,7 @@ int build_adjacency(AvbdContext *ctx, bool deviceCounts = false)
     if (T == 0)
     {
         CU(cudaMemsetAsync(ctx->adjStart.p, 0, sizeof(int) * ((size_t)n + 1), ctx->stream));
-        return build_rows<unsigned>(ctx, nullptr, 0, 0);
+        return build_rows<unsigned>(ctx, nullptr, nullptr, 0, 0);
     }
     if (T > (long long)ADJ_INDEX_MASK)
         return fail(ctx, AVBD_ERR_CAPACITY, "too many force incidences (%lld)", T);
@@ -709,11 +744,7 @@ int build_adjacency(AvbdContext *ctx, bool deviceCounts = false)
         CU(cub::DeviceRadixSort::SortPairs(ctx->cubTemp.p, bytes, dk, dv, (int)T, 0, endBit, ctx->stream));
         ctx->launches++;
         ctx->incShift = 0;
-        k_segment_starts<<<grid_for(T, 256), 256, 0, ctx->stream>>>(dk.Current(), (int)T, 0, n, ctx->adjStart.p, st);
-        LAUNCHED();
-        k_copy_adj<<<grid_for(T, 256), 256, 0, ctx->stream>>>(dv.Current(), ctx->adj.p, (int)T, st);
-        LAUNCHED();
-        return build_rows(ctx, dk.Current(), (int)T, mans, st);
+        return build_rows(ctx, dk.Current(), dv.Current(), (int)T, mans, st);
     }
     CHECK(reserve(ctx, ctx->incKeys, T, false));
     CHECK(reserve(ctx, ctx->incKeysAlt, T, false));
@@ -735,17 +766,15 @@ int build_adjacency(AvbdContext *ctx, bool deviceCounts = false)
     CHECK(ensure_temp(ctx, bytes));
     CU(cub::DeviceRadixSort::SortPairs(ctx->cubTemp.p, bytes, dk, dv, (int)T, 0, endBit, ctx->stream));
     ctx->launches++;
-    k_segment_starts<<<grid_for(T, 256), 256, 0, ctx->stream>>>(dk.Current(), (int)T, shift, n, ctx->adjStart.p, st);
-    LAUNCHED();
-    k_copy_adj<<<grid_for(T, 256), 256, 0, ctx->stream>>>(dv.Current(), ctx->adj.p, (int)T, st);
-    LAUNCHED();
-    return build_rows(ctx, dk.Current(), (int)T, mans, st);
+    return build_rows(ctx, dk.Current(), dv.Current(), (int)T, mans, st);
 }
 
-// The primal's row list, one (entry, row) pair per constraint row in force order, for the
-// dynamic bodies (no host read: sized by an upper bound, ranges from a device scan).
+// The force lists from the sorted incidences, and the primal's row list, one (entry, row) pair
+// per constraint row in force order, for the dynamic bodies (no host read: sized by an upper
+// bound, ranges from a device scan).
 template <class Key>
-int build_rows(AvbdContext *ctx, const Key *sortedKeys, int total, size_t manifolds, const StepState *st)
+int build_rows(AvbdContext *ctx, const Key *sortedKeys, const unsigned *sortedVals, int total, size_t manifolds,
+               const StepState *st)
 {
     int n = ctx->n;
     CHECK(reserve(ctx, ctx->rowStart, (size_t)n + 1, false));
@@ -759,16 +788,23 @@ int build_rows(AvbdContext *ctx, const Key *sortedKeys, int total, size_t manifo
     size_t bound = 16 * manifolds + 6 * (size_t)ctx->nJoint + 2 * (size_t)ctx->nSpring;
     CHECK(reserve(ctx, ctx->rows, std::max<size_t>(bound, 1), false));
     DevForces F = dev_forces(ctx);
-    k_entry_rows<<<grid_for((long long)total + 1, 256), 256, 0, ctx->stream>>>(F, dev_bodies(ctx), sortedKeys, total,
-                                                                               ctx->incShift, ctx->rowCount.p, st);
+    k_force_lists<<<grid_for((long long)total + 1, 256), 256, 0, ctx->stream>>>(
+        F, dev_bodies(ctx), sortedKeys, sortedVals, total, ctx->incShift, ctx->adjStart.p, ctx->adj.p, ctx->rowCount.p,
+        st);
     LAUNCHED();
-    CHECK(scan_counts(ctx, ctx->rowCount.p, ctx->entryRow.p, total + 1, 0));
-    ctx->launches++;
-    k_row_starts<<<grid_for((long long)n + 1, 256), 256, 0, ctx->stream>>>(ctx->adjStart.p, ctx->entryRow.p, n,
-                                                                           ctx->rowStart.p, st);
-    LAUNCHED();
-    F = dev_forces(ctx);
-    k_entry_fill<<<grid_for(total, 256), 256, 0, ctx->stream>>>(F, ctx->entryRow.p, ctx->rowCount.p, total, st);
+    if (total < SCAN_SMALL)
+    {
+        k_row_scan<<<1, SCAN_BLOCK, 0, ctx->stream>>>(ctx->rowCount.p, ctx->entryRow.p, total,
+                                                      ctx->nJoint + ctx->nSpring + ctx->nIgnore, st);
+        LAUNCHED();
+    }
+    else
+    {
+        CHECK(scan_counts(ctx, ctx->rowCount.p, ctx->entryRow.p, total + 1, 0));
+        ctx->launches++;
+    }
+    k_entry_fill<<<grid_for(std::max(total, n + 1), 256), 256, 0, ctx->stream>>>(F, ctx->entryRow.p, ctx->rowCount.p,
+                                                                                total, n, ctx->rowStart.p, st);
     LAUNCHED();
     return AVBD_OK;
 }
@@ -837,9 +873,8 @@ int large_cell_lists(AvbdContext *ctx, int nL, cudaStream_t s, DArr<char> &temp)
     CU(cub::DeviceRadixSort::SortKeys(temp.p, bytes, lk, total, 24, large_sort_end(ctx), s));
     ctx->launches++;
     ctx->largeSorted = lk.Current();
-    // sentinel after the sorted keys: candidate walks stop at it
-    CU(cudaMemsetAsync(lk.Current() + total, 0xFF, sizeof(unsigned long long), s));
-    CU(cudaMemsetAsync(ctx->largeHashKeys.p, 0xFF, sizeof(unsigned long long) * ((size_t)ctx->largeHashMask + 1), s));
+    // (step_clear left the hash table empty and a sentinel after either key array: candidate
+    // walks stop at it)
     k_bp_hash_large_runs<<<grid_for(total, 256), 256, 0, s>>>(lk.Current(), total, large_hash(ctx));
     LAUNCHED();
     return AVBD_OK;
@@ -915,9 +950,6 @@ int lbvh_count(AvbdContext *ctx, const unsigned long long *gridKeys, int nB, con
     return AVBD_OK;
 }
 
-// Broadphase of every world: appends new manifolds after the existing ones. `deviceCounts`
-// (grid mode only): no host read; k_bp_commit places the new pairs from the device counts
-// and the emitting passes take their base from the step state.
 // The non-finite check of a synchronous step, read after the first wait of its broadphase
 // (which has changed nothing yet): the step is refused before its new pairs are written.
 int nonfinite_checked(AvbdContext *ctx)
@@ -931,6 +963,74 @@ int nonfinite_checked(AvbdContext *ctx)
     return AVBD_OK;
 }
 
+// Slots of the pair set: a power of two, at least twice the forces it can meet.
+unsigned long long pair_set_slots(const AvbdContext *ctx, bool deviceCounts)
+{
+    const long long forces = (long long)(deviceCounts ? man_capacity(ctx) : (size_t)ctx->nMan) + ctx->nJoint +
+                             ctx->nSpring + ctx->nIgnore;
+    unsigned long long slots = 1024;
+    while (slots < 2ull * (unsigned long long)forces)
+        slots <<= 1;
+    return slots;
+}
+
+// A step's first launch: its admission check and everything the step starts from cleared
+// (k_step_begin). `seen`: the synchronous step's flags; neither a device state nor flags: the
+// clearing alone (a collision-only step; a recount, which keeps the pair set and the grid).
+int step_clear(AvbdContext *ctx, int *seen, bool deviceCounts, bool recount = false)
+{
+    StepClear C;
+    CHECK(reserve(ctx, ctx->colourCtl, 1, false));
+    CHECK(reserve(ctx, ctx->iterSync, 1, false));
+    CHECK(reserve(ctx, ctx->colourStart, 257, false));
+    C.add(ctx->counters.p, sizeof(StepCounters), 0u);
+    if (!recount)
+    {
+        C.add(ctx->colourCtl.p, sizeof(ColourControl), 0u);
+        C.add(ctx->iterSync.p, sizeof(IterSync), 0u);
+    }
+    const int mode = ctx->params.broadphase;
+    if (ctx->n >= 2 && !ctx->external && (mode == AVBD_BROADPHASE_GRID || mode == AVBD_BROADPHASE_LBVH))
+    {
+        const size_t nB = ctx->hBinned.size(), nL = ctx->hLarge.size();
+        if (!recount)
+        {
+            const size_t slots = (size_t)pair_set_slots(ctx, deviceCounts);
+            CHECK(reserve(ctx, ctx->pairSetKeys, slots, false));
+            C.add(ctx->pairSetKeys.p, sizeof(unsigned long long) * slots, ~0u);
+            C.add(ctx->cappedAny.p, sizeof(int), 0u);
+            C.bounds = ctx->bounds.p;
+            C.worlds = ctx->W;
+        }
+        if (nB)
+            C.add(ctx->cellHashKeys.p, sizeof(unsigned long long) * ((size_t)ctx->cellHashMask + 1), ~0u);
+        if (nL)
+        {
+            C.add(ctx->largeHashKeys.p, sizeof(unsigned long long) * ((size_t)ctx->largeHashMask + 1), ~0u);
+            C.add(ctx->largeKeys.p + nL * LARGE_MAX_CELLS, sizeof(unsigned long long), ~0u);
+            C.add(ctx->largeKeysAlt.p + nL * LARGE_MAX_CELLS, sizeof(unsigned long long), ~0u);
+            CHECK(reserve(ctx, ctx->llChunkLo, nL, false));
+            CHECK(reserve(ctx, ctx->llChunkHi, nL, false));
+            C.add(ctx->llChunkHi.p, sizeof(uint4) * nL, 0u);
+            C.chunkLo = ctx->llChunkLo.p;
+            C.chunks = (int)nL;
+        }
+    }
+    DevBodies B = dev_bodies(ctx);
+    StepState *st = deviceCounts ? ctx->stepState.p : nullptr;
+    if (!st && !seen)
+        B.n = 0;
+    const int J = deviceCounts ? ctx->nJoint : 0;
+    const int blocks = std::max(grid_for(std::max(std::max(B.n, J), 1), 256),
+                                std::min(grid_for(std::max(C.most / 4, 8ll * C.worlds), 256), 148 * 4));
+    k_step_begin<<<blocks, 256, 0, ctx->stream>>>(B, deviceCounts ? ctx->joint[ctx->jcur].p : nullptr, J, st, seen, C);
+    LAUNCHED();
+    return AVBD_OK;
+}
+
+// Broadphase of every world: appends new manifolds after the existing ones. `deviceCounts`
+// (grid, LBVH and sweep-and-prune modes): no host read; the commit places the new pairs from
+// the device counts and the emitting passes take their base from the step state.
 int broadphase(AvbdContext *ctx, bool deviceCounts = false)
 {
     int n = ctx->n;
@@ -1057,16 +1157,11 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
         PairSet S;
         const long long forces = (long long)(deviceCounts ? man_capacity(ctx) : (size_t)ctx->nMan) + ctx->nJoint +
                                  ctx->nSpring + ctx->nIgnore;
-        unsigned long long slots = 1024;
-        while (slots < 2ull * (unsigned long long)forces)
-            slots <<= 1;
-        CHECK(reserve(ctx, ctx->pairSetKeys, (size_t)slots, false));
-        S.keys = ctx->pairSetKeys.p;
-        S.mask = (unsigned)(slots - 1);
+        S.keys = ctx->pairSetKeys.p; // reserved and cleared by step_clear
+        S.mask = (unsigned)(pair_set_slots(ctx, deviceCounts) - 1);
+        const bool scanInCommit = deviceCounts && nB <= SCAN_SMALL && nItems <= SCAN_SMALL;
         if (nItems > 0)
         {
-            CHECK(reserve(ctx, ctx->llChunkLo, (size_t)nL, false));
-            CHECK(reserve(ctx, ctx->llChunkHi, (size_t)nL, false));
             CHECK(reserve(ctx, ctx->llRecorded, (size_t)nItems * LL_SLOTS, false));
             size_t bytes = 0;
             cub::DeviceScan::ExclusiveSum(nullptr, bytes, ctx->llCount.p, ctx->llOffset.p, nItems);
@@ -1086,8 +1181,6 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
         auto large_large_count = [&](cudaStream_t s) -> int {
             if (nItems > 0)
             {
-                k_ll_chunk_init<<<grid_for(nL, 256), 256, 0, s>>>(ctx->llChunkLo.p, ctx->llChunkHi.p, nL);
-                LAUNCHED();
                 k_ll_chunk_bounds<<<grid_for(nL, 128), 128, 0, s>>>(G, ctx->large.p, ctx->largeSphere.p, nL,
                                                                     ctx->llChunkLo.p, ctx->llChunkHi.p);
                 LAUNCHED();
@@ -1095,6 +1188,8 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
                     F, ctx->large.p, ctx->largeSphere.p, ctx->llItems.p, nItems, ctx->llCount.p, nullptr, 0, 0, cnt,
                     nullptr, ctx->llChunkLo.p, ctx->llChunkHi.p, ctx->llRecorded.p, S);
                 LAUNCHED();
+                if (scanInCommit)
+                    return AVBD_OK;
                 size_t bytes = ctx->cubTempSide[0].cap;
                 CU(cub::DeviceScan::ExclusiveSum(ctx->cubTempSide[0].p, bytes, ctx->llCount.p, ctx->llOffset.p, nItems,
                                                  s));
@@ -1123,8 +1218,6 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
             CHECK(ensure_temp(ctx, bytes));
             CU(cub::DeviceRadixSort::SortKeys(ctx->cubTemp.p, bytes, dk, nB, 24, gridEnd, M));
             ctx->launches++;
-            CU(cudaMemsetAsync(ctx->cellHashKeys.p, 0xFF,
-                               sizeof(unsigned long long) * ((size_t)ctx->cellHashMask + 1), M));
             k_bp_hash_runs<<<grid_for(nB, 256), 256, 0, M>>>(dk.Current(), nB, cell_hash(ctx));
             LAUNCHED();
             CHECK(reserve(ctx, ctx->pairRecorded, (size_t)nB * BP_LANES * BP_SLOTS, false));
@@ -1143,6 +1236,8 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
                 CU(cudaStreamWaitEvent(M, evTree, 0)); // the tree, built on side[3]
                 CHECK(lbvh_count(ctx, dk.Current(), nB, S));
             }
+            if (scanInCommit)
+                return AVBD_OK;
             CHECK(scan_counts(ctx, ctx->pairCount.p, ctx->pairOffset.p, nB, 0));
             ctx->launches++;
             if (!deviceCounts)
@@ -1155,27 +1250,18 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
         // side[0]: pair set, large boxes, large-large pass
         CU(cudaEventRecord(evFork, M));
         CU(cudaStreamWaitEvent(S1, evFork, 0));
-        CU(cudaMemsetAsync(ctx->pairSetKeys.p, 0xFF, sizeof(unsigned long long) * slots, S1));
-        k_pair_set<<<grid_for(std::max(forces, 1ll), 256), 256, 0, S1>>>(dev_forces(ctx), S, stp);
+        k_pair_set_large<<<grid_for(std::max(std::max(forces, (long long)nL), 1ll), 256), 256, 0, S1>>>(
+            dev_forces(ctx), S, stp, B, ctx->large.p, nL, dt, ctx->largeLo.p, ctx->largeHi.p, ctx->largeSphere.p);
         LAUNCHED();
         CU(cudaEventRecord(evPairSet, S1));
-        if (nL)
-        {
-            k_bp_large<<<grid_for(nL, 64), 64, 0, S1>>>(B, ctx->large.p, nL, dt, ctx->largeLo.p, ctx->largeHi.p,
-                                                        ctx->largeSphere.p);
-            LAUNCHED();
-        }
         CU(cudaEventRecord(evLarge, S1));
         CHECK(large_large_count(S1));
         CU(cudaEventRecord(evLL, S1));
         // context stream: bounds and grid parameters, then (side[1]) the large cell lists
         // beside the grid entries' sort
-        CU(cudaMemsetAsync(ctx->cappedAny.p, 0, sizeof(int), M));
         ctx->largeSorted = ctx->largeKeys.p;
         if (nB)
         {
-            k_bp_bounds_init<<<grid_for(8ll * ctx->W, 256), 256, 0, M>>>(ctx->bounds.p, ctx->W);
-            LAUNCHED();
             k_bp_bounds<<<std::min(grid_for(nB, 256), 148 * 2), 256, 0, M>>>(B, G, ctx->binned.p, nB, dt);
             LAUNCHED();
             k_bp_params<<<grid_for(ctx->W, 128), 128, 0, M>>>(G, ctx->worldBinned.p);
@@ -1201,24 +1287,25 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
         if (deviceCounts)
         {
             StepState *st = ctx->stepState.p;
-            k_bp_commit<<<1, 1, 0, ctx->stream>>>(st, ctx->pairOffset.p, ctx->pairCount.p, nB, ctx->llOffset.p,
-                                                  ctx->llCount.p, nItems, ctx->cappedAny.p, cnt,
-                                                  (long long)man_capacity(ctx));
+            if (scanInCommit)
+                k_bp_scan_commit<<<1, SCAN_BLOCK, 0, ctx->stream>>>(
+                    st, ctx->pairOffset.p, ctx->pairCount.p, nB, ctx->llOffset.p, ctx->llCount.p, nItems,
+                    ctx->cappedAny.p, cnt, (long long)man_capacity(ctx));
+            else
+                k_bp_commit<<<1, 1, 0, ctx->stream>>>(st, ctx->pairOffset.p, ctx->pairCount.p, nB, ctx->llOffset.p,
+                                                      ctx->llCount.p, nItems, ctx->cappedAny.p, cnt,
+                                                      (long long)man_capacity(ctx));
             LAUNCHED();
             F = dev_forces(ctx);
-            if (nB)
+            const int entryBlocks = nB ? grid_for((long long)nB * BP_LANES, 128) : 0;
+            const int llBlocks = nItems > 0 ? grid_for(nItems, 128) : 0;
+            if (entryBlocks + llBlocks > 0)
             {
-                k_bp_pairs<BP_EMIT_RECORDED><<<grid_for((long long)nB * BP_LANES, 128), 128, 0, ctx->stream>>>(
+                k_bp_emit<<<entryBlocks + llBlocks, 128, 0, ctx->stream>>>(
                     B, F, G, dk.Current(), nB, cell_hash(ctx), ctx->large.p, ctx->largeLo.p, ctx->largeHi.p,
-                    ctx->largeSorted, large_hash(ctx), dt, ctx->pairCount.p, ctx->pairOffset.p, 0, 0, cnt,
-                    ctx->pairRecorded.p, ctx->pairLaneCount.p, st, S);
-                LAUNCHED();
-            }
-            if (nItems > 0)
-            {
-                k_bp_large_large<BP_EMIT_RECORDED><<<grid_for(nItems, 128), 128, 0, ctx->stream>>>(
-                    F, ctx->large.p, ctx->largeSphere.p, ctx->llItems.p, nItems, ctx->llCount.p, ctx->llOffset.p, 0, 0,
-                    cnt, st, ctx->llChunkLo.p, ctx->llChunkHi.p, ctx->llRecorded.p, S);
+                    ctx->largeSorted, large_hash(ctx), dt, ctx->pairCount.p, ctx->pairOffset.p, cnt,
+                    ctx->pairRecorded.p, ctx->pairLaneCount.p, st, S, entryBlocks, ctx->largeSphere.p, ctx->llItems.p,
+                    nItems, ctx->llCount.p, ctx->llOffset.p, ctx->llChunkLo.p, ctx->llChunkHi.p, ctx->llRecorded.p);
                 LAUNCHED();
             }
             return AVBD_OK;
@@ -1238,7 +1325,7 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
                     host_grid_cap(ctx->hGrid[w]);
             CU(cudaMemcpyAsync(ctx->grid.p, ctx->hGrid, sizeof(GridParams) * ctx->W, cudaMemcpyHostToDevice,
                                ctx->stream));
-            CU(cudaMemsetAsync(cnt, 0, sizeof(StepCounters), ctx->stream));
+            CHECK(step_clear(ctx, nullptr, false, true));
             // the recount runs on the context stream alone (every side stream has joined)
             if (nL)
                 CHECK(large_cell_lists(ctx, nL, M, ctx->cubTempSide[1]));
@@ -1345,19 +1432,27 @@ int init_forces_device(AvbdContext *ctx)
             k_manifold_init<false><<<grid_for(M, 128), 128, 0, ctx->stream>>>(
                 B, Md, M, P, ctx->keep.p, st, ExternalContacts(), orphans, Mo, INIT_NEW);
         LAUNCHED();
-        k_u8_to_int<<<grid_for(M, 256), 256, 0, ctx->stream>>>(ctx->keep.p, cnt32, M, st);
-        LAUNCHED();
-        CHECK(scan_counts(ctx, cnt32, idx, M, 0));
-        ctx->launches++;
-        // back into the live buffer: no swap
-        k_manifold_compact<<<grid_for((long long)M * COMPACT_LANES, 128), 128, 0, ctx->stream>>>(
-            Mo, Md, M, ctx->keep.p, idx, st, false, dev_forces(ctx).contactFlow);
-        LAUNCHED();
+        if (M <= SCAN_SMALL)
+        {
+            k_keep_scan<<<1, SCAN_BLOCK, 0, ctx->stream>>>(ctx->keep.p, idx, M, st);
+            LAUNCHED();
+        }
+        else
+        {
+            k_u8_to_int<<<grid_for(M, 256), 256, 0, ctx->stream>>>(ctx->keep.p, cnt32, M, st);
+            LAUNCHED();
+            CHECK(scan_counts(ctx, cnt32, idx, M, 0));
+            ctx->launches++;
+        }
     }
-    if (J)
+    if (M || J)
     {
+        // back into the live buffer: no swap
+        DevManifolds Md = dev_man(ctx->man[ctx->cur]), Mo = dev_man(ctx->man[ctx->cur ^ 1]);
         DevForces F = dev_forces(ctx);
-        k_joint_init<<<grid_for(J, 128), 128, 0, ctx->stream>>>(B, F, P, ctx->keep.p, st, &ctx->counters.p->orphans);
+        const int blocks = grid_for((long long)M * COMPACT_LANES, 128) + (J ? grid_for(J, 128) : 0);
+        k_forces_commit<<<blocks, 128, 0, ctx->stream>>>(Mo, Md, M, ctx->keep.p, idx, st, F.contactFlow, B, F, P,
+                                                         &ctx->counters.p->orphans);
         LAUNCHED();
     }
     return AVBD_OK;
@@ -1490,7 +1585,7 @@ int init_forces(AvbdContext *ctx)
         CHECK(reserve_manifolds(ctx, dst, (size_t)std::max<long long>(newM, 1), 0));
         CHECK(flow_reserve(ctx, (size_t)newM));
         k_manifold_compact<<<grid_for((long long)M * COMPACT_LANES, 128), 128, 0, ctx->stream>>>(
-            Md, dev_man(dst), M, ctx->keep.p, idx, nullptr, true, dev_forces(ctx).contactFlow);
+            Md, dev_man(dst), M, ctx->keep.p, idx, dev_forces(ctx).contactFlow);
         LAUNCHED();
         ctx->cur ^= 1;
         ctx->nMan = (int)newM;
@@ -1499,8 +1594,7 @@ int init_forces(AvbdContext *ctx)
     {
         CHECK(flow_reserve(ctx, 0));
         DevForces F = dev_forces(ctx);
-        k_joint_init<<<grid_for(J, 128), 128, 0, ctx->stream>>>(B, F, P, ctx->keep.p, nullptr,
-                                                                 &ctx->counters.p->orphans);
+        k_joint_init<<<grid_for(J, 128), 128, 0, ctx->stream>>>(B, F, P, ctx->keep.p, &ctx->counters.p->orphans);
         LAUNCHED();
         k_u8_to_int<<<grid_for(J, 256), 256, 0, ctx->stream>>>(ctx->keep.p, cnt32, J);
         LAUNCHED();
@@ -1557,7 +1651,6 @@ int colour_bodies(AvbdContext *ctx, bool deviceCounts = false)
         ctx->hColourStart.assign(1, 0);
         return AVBD_OK;
     }
-    CU(cudaMemsetAsync(ctx->colourCtl.p, 0, sizeof(ColourControl), ctx->stream));
     int blocks = std::min(grid_for(std::max(n, 1), 256), ctx->colourBlocks);
     int mode = ctx->colourMode;
     unsigned spinLimit = ctx->waitColour ? ctx->waitColour : BARRIER_SPIN_LIMIT;
@@ -1658,8 +1751,6 @@ int iterate_persistent(AvbdContext *ctx, bool deviceCounts = false, IterTape tap
     DevBodies B = dev_bodies(ctx);
     DevForces F = dev_forces(ctx);
     Params P = dev_params(ctx->params);
-    CHECK(reserve(ctx, ctx->iterSync, 1, false));
-    CU(cudaMemsetAsync(ctx->iterSync.p, 0, sizeof(IterSync), ctx->stream));
     int nColours = ctx->nColours, iterations = ctx->params.iterations;
     const int4 *entries = ctx->solveEntry.p;
     const int *colourStart = ctx->colourStart.p;
@@ -1758,9 +1849,7 @@ int step_once(AvbdContext *ctx)
 {
     // refuse non-finite body state before anything changes, like a device-resident step
     CU(cudaMemsetAsync(ctx->stepFlags.p, 0, sizeof(int), ctx->stream));
-    k_step_begin<<<grid_for(std::max(ctx->n, 1), 256), 256, 0, ctx->stream>>>(dev_bodies(ctx), nullptr, 0, nullptr,
-                                                                               ctx->stepFlags.p);
-    LAUNCHED();
+    CHECK(step_clear(ctx, ctx->stepFlags.p, false));
     CU(cudaMemcpyAsync(ctx->hStepFlags, ctx->stepFlags.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     ctx->flagsPending = true; // read by the broadphase at its wait for the pair counts
     if (ctx->recording)
@@ -1772,7 +1861,6 @@ int step_once(AvbdContext *ctx)
             return rc;
         }
     }
-    CU(cudaMemsetAsync(ctx->counters.p, 0, sizeof(StepCounters), ctx->stream));
     ctx->stats.grid_rescaled = 0;
     {
         PhaseScope ps(ctx, AVBD_PHASE_BROADPHASE);
@@ -1846,6 +1934,8 @@ int push_state(AvbdContext *ctx)
     ctx->flipsAtConfirm = 0;
     ctx->curAtConfirm = ctx->cur;
     ctx->seqBound = (unsigned long long)ctx->nextSeq;
+    ctx->stateMan = ctx->nMan;
+    ctx->stateSeq = ctx->nextSeq;
     ctx->stateDirty = false;
     return AVBD_OK;
 }
@@ -1882,23 +1972,20 @@ int step_device(AvbdContext *ctx)
 {
     // with no step pending the host's counts are current (a settle, a synchronous step, a
     // load or an edit came last): they become the device state's
-    if (ctx->stateDirty || ctx->pendingFast == 0)
+    if (ctx->stateDirty || (ctx->pendingFast == 0 && (ctx->nMan != ctx->stateMan || ctx->nextSeq != ctx->stateSeq ||
+                                                      ctx->cur != ctx->curAtConfirm)))
         CHECK(push_state(ctx));
     CHECK(device_reserve(ctx));
     // this step's new manifolds take sequence numbers below nextSeq + capacity: the bound the
     // incidence keys of this step (and of later pending steps) are sized by
     ctx->seqBound += (unsigned long long)man_capacity(ctx);
     StepState *st = ctx->stepState.p;
-    CU(cudaMemsetAsync(ctx->counters.p, 0, sizeof(StepCounters), ctx->stream));
     ctx->stats.grid_rescaled = 0;
     DevBodies B = dev_bodies(ctx);
     Params P = dev_params(ctx->params);
     {
         PhaseScope ps(ctx, AVBD_PHASE_BROADPHASE);
-        const int J = ctx->nJoint;
-        k_step_begin<<<grid_for(std::max(std::max(ctx->n, J), 1), 256), 256, 0, ctx->stream>>>(
-            B, ctx->joint[ctx->jcur].p, J, st, nullptr);
-        LAUNCHED();
+        CHECK(step_clear(ctx, nullptr, true));
         CHECK(init_old_manifolds(ctx));
         CHECK(broadphase(ctx, true));
     }
@@ -1933,13 +2020,9 @@ int step_device(AvbdContext *ctx)
             LAUNCHED();
         }
     }
-    k_step_end<<<1, 1, 0, ctx->stream>>>(st, ctx->iterSync.p);
+    k_step_end<<<1, 288, 0, ctx->stream>>>(st, ctx->iterSync.p, ctx->counters.p, ctx->colourStart.p, ctx->hState,
+                                           ctx->hCounters, ctx->hColourStarts);
     LAUNCHED();
-    CU(cudaMemcpyAsync(ctx->hState, st, sizeof(StepState), cudaMemcpyDeviceToHost, ctx->stream));
-    CU(cudaMemcpyAsync(ctx->hCounters, ctx->counters.p, sizeof(StepCounters), cudaMemcpyDeviceToHost, ctx->stream));
-    // the colour ranges, for host-side users of the last colouring (per-colour launches)
-    CU(cudaMemcpyAsync(ctx->hColourStarts, ctx->colourStart.p, sizeof(int) * 257, cudaMemcpyDeviceToHost,
-                       ctx->stream));
     ctx->pendingFast++;
     ctx->deviceSteps++;
     if (ctx->profiling)
@@ -1971,6 +2054,8 @@ int settle(AvbdContext *ctx)
     ctx->flipsAtConfirm = s.flips;
     ctx->curAtConfirm = ctx->cur;
     ctx->seqBound = s.nextSeq;
+    ctx->stateMan = ctx->nMan;
+    ctx->stateSeq = ctx->nextSeq;
     if (done > 0)
     {
         ctx->hColourStart.assign(ctx->hColourStarts, ctx->hColourStarts + std::min(std::max(ctx->nColours, 0), 256) + 1);
@@ -2374,6 +2459,82 @@ int classify_bodies(AvbdContext *ctx, const float *radius)
 
 } // namespace
 
+namespace
+{
+
+// The iteration kernels' dynamic shared memory (set per context created: a reset of the device
+// by its owner forgets it).
+bool allow_iteration_smem()
+{
+    const struct { const void *kernel; size_t bytes; } wanted[] = {
+        {(const void *)k_iterations<ITER_G, ITER_BLOCK, ITER_SUB, false>, sizeof(PrimalShared<ITER_G, ITER_BLOCK>)},
+        {(const void *)k_iterations<ITER_G, ITER_BLOCK, ITER_SUB, true>, sizeof(PrimalShared<ITER_G, ITER_BLOCK>)},
+        {(const void *)k_iterations<ITER_G, ITER_BLOCK, ITER_SUB, false, true>, sizeof(PrimalShared<ITER_G, ITER_BLOCK>)},
+        {(const void *)k_iterations_wide<false, false>, sizeof(WideShared)},
+        {(const void *)k_iterations_wide<true, false>, sizeof(WideShared)},
+        {(const void *)k_iterations_wide<false, true>, sizeof(WideShared)},
+    };
+    bool ok = true;
+    for (const auto &w : wanted)
+        ok = cudaFuncSetAttribute(w.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)w.bytes) == cudaSuccess && ok;
+    cudaGetLastError(); // an unsupported configuration only leaves the per-colour launches
+    return ok;
+}
+
+// Co-resident blocks of the cooperative kernels, the same for every context of a device: asked
+// for once per device (the occupancy queries are a good part of a small world's creation).
+struct LaunchShape
+{
+    int colourBlocks = 1, colourFlowBlocks = 1, iterBlocks = 0, wideBlocks = 0;
+};
+
+LaunchShape query_launch_shape(int device_ordinal, bool iterations)
+{
+    LaunchShape shape;
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_ordinal);
+    auto per_sm = [](const void *kernel, int block, size_t smem) {
+        int blocks = 0;
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, block, smem) == cudaSuccess ? blocks : 0;
+    };
+    shape.colourBlocks = std::max(1, sms * std::max(1, per_sm((const void *)k_colour_all, 256, 0)));
+    // the greedy colouring: co-resident, and at most four blocks per SM (every block
+    // reads all blocks' colour counts once; more resident warps mean fewer grid-stride
+    // batches per warp, which a chain of neighbours crosses one after another)
+    shape.colourFlowBlocks =
+        std::max(1, sms * std::min(4, std::max(1, per_sm((const void *)k_colour_greedy, COLOUR_FLOW_BLOCK, 0))));
+    if (iterations)
+    {
+        const size_t smem = sizeof(PrimalShared<ITER_G, ITER_BLOCK>);
+        shape.iterBlocks =
+            sms * std::min({per_sm((const void *)k_iterations<ITER_G, ITER_BLOCK, ITER_SUB, false>, ITER_BLOCK, smem),
+                            per_sm((const void *)k_iterations<ITER_G, ITER_BLOCK, ITER_SUB, true>, ITER_BLOCK, smem),
+                            per_sm((const void *)k_iterations<ITER_G, ITER_BLOCK, ITER_SUB, false, true>, ITER_BLOCK,
+                                   smem)});
+        const int wide =
+            std::min({per_sm((const void *)k_iterations_wide<false, false>, WIDE_BLOCK, sizeof(WideShared)),
+                      per_sm((const void *)k_iterations_wide<true, false>, WIDE_BLOCK, sizeof(WideShared)),
+                      per_sm((const void *)k_iterations_wide<false, true>, WIDE_BLOCK, sizeof(WideShared))});
+        shape.wideBlocks = wide > 0 ? sms : 0;
+    }
+    cudaGetLastError();
+    return shape;
+}
+
+LaunchShape launch_shape(int device)
+{
+    const bool iterations = allow_iteration_smem();
+    static std::mutex lock;
+    static std::map<int, LaunchShape> known;
+    std::lock_guard<std::mutex> hold(lock);
+    auto it = known.find(device);
+    if (it == known.end())
+        it = known.emplace(device, query_launch_shape(device, iterations)).first;
+    return it->second;
+}
+
+} // namespace
+
 extern "C"
 {
 
@@ -2446,47 +2607,11 @@ int avbd_create(AvbdContext **out, int32_t device_ordinal, void *cuda_stream)
     memset(ctx->hCounters, 0, sizeof(StepCounters));
     memset(ctx->hState, 0, sizeof(StepState));
     *ctx->hIterError = 0;
-    {
-        int sms = 0, perSm = 0;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_ordinal);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_colour_all, 256, 0);
-        ctx->colourBlocks = std::max(1, sms * std::max(1, perSm));
-        // the greedy colouring: co-resident, and at most four blocks per SM (every block
-        // reads all blocks' colour counts once; more resident warps mean fewer grid-stride
-        // batches per warp, which a chain of neighbours crosses one after another)
-        int flowSm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&flowSm, k_colour_greedy, COLOUR_FLOW_BLOCK, 0);
-        ctx->colourFlowBlocks = std::max(1, sms * std::min(4, std::max(1, flowSm)));
-        // the iteration kernel: one block of ITER_BLOCK threads per SM with its shared batch
-        int iterSm = 0;
-        size_t smem = sizeof(PrimalShared<ITER_G, ITER_BLOCK>);
-        int roundSm = 0, tapeSm = 0;
-        if (cudaFuncSetAttribute((const void *)k_iterations<ITER_G, ITER_BLOCK, ITER_SUB, false>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
-            cudaFuncSetAttribute((const void *)k_iterations<ITER_G, ITER_BLOCK, ITER_SUB, true>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
-            cudaFuncSetAttribute((const void *)k_iterations<ITER_G, ITER_BLOCK, ITER_SUB, false, true>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&tapeSm, k_iterations<ITER_G, ITER_BLOCK, ITER_SUB, false, true>,
-                                                          ITER_BLOCK, smem) == cudaSuccess &&
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&iterSm, k_iterations<ITER_G, ITER_BLOCK, ITER_SUB, false>,
-                                                          ITER_BLOCK, smem) == cudaSuccess &&
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&roundSm, k_iterations<ITER_G, ITER_BLOCK, ITER_SUB, true>,
-                                                          ITER_BLOCK, smem) == cudaSuccess)
-            ctx->iterBlocks = sms * std::min({iterSm, roundSm, tapeSm});
-        // the wide form, for narrow worlds
-        int wideSm[3] = {0, 0, 0};
-        const void *wide[3] = {(const void *)k_iterations_wide<false, false>, (const void *)k_iterations_wide<true, false>,
-                               (const void *)k_iterations_wide<false, true>};
-        for (int k = 0; k < 3; ++k)
-            if (cudaFuncSetAttribute(wide[k], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WideShared)) !=
-                    cudaSuccess ||
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&wideSm[k], wide[k], WIDE_BLOCK, sizeof(WideShared)) !=
-                    cudaSuccess)
-                wideSm[k] = 0;
-        ctx->wideBlocks = std::min({wideSm[0], wideSm[1], wideSm[2]}) > 0 ? sms : 0;
-        cudaGetLastError(); // an unsupported configuration only leaves the per-colour launches
-    }
+    const LaunchShape shape = launch_shape(device_ordinal);
+    ctx->colourBlocks = shape.colourBlocks;
+    ctx->colourFlowBlocks = shape.colourFlowBlocks;
+    ctx->iterBlocks = shape.iterBlocks;
+    ctx->wideBlocks = shape.wideBlocks;
     if (reserve(ctx, ctx->counters, 1, false) || reserve(ctx, ctx->bounds, 8, false) ||
         reserve(ctx, ctx->grid, 1, false) || reserve(ctx, ctx->stepState, 1, false) ||
         reserve(ctx, ctx->stepFlags, 1, false))
@@ -3090,7 +3215,7 @@ int avbd_broadphase_only(AvbdContext *ctx)
     // joints, springs and ignore pairs count as constraints for the broadphase
     ctx->nMan = 0;
     CHECK(build_adjacency(ctx));
-    CU(cudaMemsetAsync(ctx->counters.p, 0, sizeof(StepCounters), ctx->stream));
+    CHECK(step_clear(ctx, nullptr, false));
     ctx->stats.grid_rescaled = 0;
     {
         PhaseScope ps(ctx, AVBD_PHASE_BROADPHASE);

@@ -254,12 +254,11 @@ AVBD_DEV bool linked(const DevForces &F, const PairSet &S, int a, int b)
     return S.keys ? pair_linked(S, a, b) : constrained(F, a, b);
 }
 
-// One thread per force (manifolds, joints, springs, ignore pairs): insert its body pair.
-__global__ void k_pair_set(DevForces F, PairSet S, const StepState *st = nullptr)
+// Force f (manifolds, joints, springs, ignore pairs): insert its body pair.
+AVBD_DEV void pair_set_insert(DevForces F, const PairSet &S, int f, const StepState *st)
 {
     if (st)
         F.nMan = st->nMan;
-    int f = blockIdx.x * blockDim.x + threadIdx.x;
     int2 ab;
     if (f < F.nMan)
         ab = F.man.ab[f];
@@ -372,15 +371,6 @@ AVBD_DEV unsigned float_order(float f)
 }
 AVBD_DEV float float_unorder(unsigned u) { return __uint_as_float((u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u); }
 
-__global__ void k_bp_bounds_init(unsigned *bounds, int W)
-{
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= 8 * W)
-        return;
-    int slot = k & 7;
-    bounds[k] = slot < 3 ? 0xFFFFFFFFu : 0u; // min slots, then max slots and the largest binned slack
-}
-
 // Bounds of each world's binned centres and its largest binned travel slack
 // (solver.cpp:306-333). Each thread folds its grid-stride items while they stay in one world
 // (bodies of a world are contiguous in the binned list), then warps and the block combine
@@ -477,12 +467,8 @@ __global__ void __launch_bounds__(256) k_bp_bounds(DevBodies B, DevGrid G, const
 }
 
 // World AABB plus travel slack of the bodies too large for the grid (solver.cpp:311-327)
-__global__ void k_bp_large(DevBodies B, const int *large, int nLarge, float dt, float4 *lo, float4 *hi,
-                           float4 *sphere)
+AVBD_DEV void large_box(const DevBodies &B, int k, const int *large, float dt, float4 *lo, float4 *hi, float4 *sphere)
 {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nLarge)
-        return;
     int b = large[k];
     float3 p = xyz(B.pos[b]);
     float4 q = B.quat[b];
@@ -502,6 +488,16 @@ __global__ void k_bp_large(DevBodies B, const int *large, int nLarge, float dt, 
     lo[k] = f4(sub(p, h), slack);
     hi[k] = f4(add(p, h), slack);
     sphere[k] = f4(p, sr.w);
+}
+
+// The pair set and the large bodies' boxes (independent of one another: one launch).
+__global__ void k_pair_set_large(DevForces F, PairSet S, const StepState *st, DevBodies B, const int *large, int nLarge,
+                                 float dt, float4 *lo, float4 *hi, float4 *sphere)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    pair_set_insert(F, S, t, st);
+    if (t < nLarge)
+        large_box(B, t, large, dt, lo, hi, sphere);
 }
 
 // Cell size and grid dimensions per world (solver.cpp:338-357). When the cell count
@@ -684,17 +680,14 @@ constexpr unsigned BP_UNRECORDED = 1u << 30; // lane count flag: its partners we
 constexpr int BP_LANES = 16; // lanes per grid entry (15 parts)
 
 template <int MODE>
-__global__ void __launch_bounds__(128) k_bp_pairs(DevBodies B, DevForces F, DevGrid G, const unsigned long long *keys,
-                                                  int nBinned, HashTable cells, const int *large,
-                                                  const float4 *largeLo, const float4 *largeHi,
-                                                  const unsigned long long *largeKeys, HashTable largeCells, float dt,
-                                                  int *counts, const int *offsets, int base, unsigned long long seqBase,
-                                                  StepCounters *cnt, int *recorded, int *laneCounts,
-                                                  const StepState *st = nullptr, PairSet S = PairSet(),
-                                                  unsigned partMask = 0x7FFFu)
+AVBD_DEV void bp_pairs(long long tid, const DevBodies &B, const DevForces &F, const DevGrid &G,
+                       const unsigned long long *keys, int nBinned, HashTable cells, const int *large,
+                       const float4 *largeLo, const float4 *largeHi, const unsigned long long *largeKeys,
+                       HashTable largeCells, float dt, int *counts, const int *offsets, int base,
+                       unsigned long long seqBase, StepCounters *cnt, int *recorded, int *laneCounts,
+                       const StepState *st, PairSet S, unsigned partMask)
 {
     constexpr bool EMIT = MODE != BP_COUNT;
-    const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int i = (int)(tid / BP_LANES);
     const int part = (int)(tid % BP_LANES);
     const bool entry = i < nBinned;
@@ -868,6 +861,21 @@ __global__ void __launch_bounds__(128) k_bp_pairs(DevBodies B, DevForces F, DevG
         warp_add(&cnt->sphereHits, hits);
         warp_add(&cnt->constrainedHits, cons);
     }
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(128) k_bp_pairs(DevBodies B, DevForces F, DevGrid G, const unsigned long long *keys,
+                                                  int nBinned, HashTable cells, const int *large,
+                                                  const float4 *largeLo, const float4 *largeHi,
+                                                  const unsigned long long *largeKeys, HashTable largeCells, float dt,
+                                                  int *counts, const int *offsets, int base, unsigned long long seqBase,
+                                                  StepCounters *cnt, int *recorded, int *laneCounts,
+                                                  const StepState *st = nullptr, PairSet S = PairSet(),
+                                                  unsigned partMask = 0x7FFFu)
+{
+    bp_pairs<MODE>((long long)blockIdx.x * blockDim.x + threadIdx.x, B, F, G, keys, nBinned, cells, large, largeLo,
+                   largeHi, largeKeys, largeCells, dt, counts, offsets, base, seqBase, cnt, recorded, laneCounts, st, S,
+                   partMask);
 }
 
 // ---------------------------------------------------------------------------
@@ -1194,16 +1202,6 @@ constexpr int LL_SLOTS = 8;
 // large body folds its sphere into its chunk's box with atomic min / max. The boxes start at
 // (all ones, 0) for the minima and 0 for the maxima; w of the minimum marks a non-finite
 // sphere in the chunk (no culling there).
-__global__ void k_ll_chunk_init(uint4 *lo, uint4 *hi, int nLarge)
-{
-    int l = blockIdx.x * blockDim.x + threadIdx.x;
-    if (l < nLarge)
-    {
-        lo[l] = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u);
-        hi[l] = make_uint4(0u, 0u, 0u, 0u);
-    }
-}
-
 __global__ void k_ll_chunk_bounds(DevGrid G, const int *large, const float4 *largeSphere, int nLarge, uint4 *lo,
                                   uint4 *hi)
 {
@@ -1229,13 +1227,12 @@ __global__ void k_ll_chunk_bounds(DevGrid G, const int *large, const float4 *lar
 }
 
 template <int MODE>
-__global__ void k_bp_large_large(DevForces F, const int *large, const float4 *largeSphere, const int4 *items,
-                                 int nItems, int *counts, const int *offsets, int base, unsigned long long seqBase,
-                                 StepCounters *cnt, const StepState *st, const uint4 *chunkLo,
-                                 const uint4 *chunkHi, int *recorded, PairSet S = PairSet())
+AVBD_DEV void bp_large_large(int w, const DevForces &F, const int *large, const float4 *largeSphere, const int4 *items,
+                             int nItems, int *counts, const int *offsets, int base, unsigned long long seqBase,
+                             StepCounters *cnt, const StepState *st, const uint4 *chunkLo, const uint4 *chunkHi,
+                             int *recorded, PairSet S)
 {
     constexpr bool EMIT = MODE != BP_COUNT;
-    const int w = blockIdx.x * blockDim.x + threadIdx.x;
     if (EMIT && st)
     {
         if (step_aborted(st))
@@ -1324,6 +1321,36 @@ __global__ void k_bp_large_large(DevForces F, const int *large, const float4 *la
         warp_add(&cnt->sphereHits, hits);
         warp_add(&cnt->constrainedHits, cons);
     }
+}
+
+template <int MODE>
+__global__ void k_bp_large_large(DevForces F, const int *large, const float4 *largeSphere, const int4 *items,
+                                 int nItems, int *counts, const int *offsets, int base, unsigned long long seqBase,
+                                 StepCounters *cnt, const StepState *st, const uint4 *chunkLo,
+                                 const uint4 *chunkHi, int *recorded, PairSet S = PairSet())
+{
+    bp_large_large<MODE>(blockIdx.x * blockDim.x + threadIdx.x, F, large, largeSphere, items, nItems, counts, offsets,
+                         base, seqBase, cnt, st, chunkLo, chunkHi, recorded, S);
+}
+
+// A device step's emission: the grid entries' new pairs, and after their blocks the large
+// bodies'.
+__global__ void __launch_bounds__(128)
+    k_bp_emit(DevBodies B, DevForces F, DevGrid G, const unsigned long long *keys, int nBinned, HashTable cells,
+              const int *large, const float4 *largeLo, const float4 *largeHi, const unsigned long long *largeKeys,
+              HashTable largeCells, float dt, int *counts, const int *offsets, StepCounters *cnt, int *recorded,
+              int *laneCounts, const StepState *st, PairSet S, int entryBlocks, const float4 *largeSphere,
+              const int4 *items, int nItems, int *llCounts, const int *llOffsets, const uint4 *chunkLo,
+              const uint4 *chunkHi, int *llRecorded)
+{
+    if ((int)blockIdx.x < entryBlocks)
+        bp_pairs<BP_EMIT_RECORDED>((long long)blockIdx.x * blockDim.x + threadIdx.x, B, F, G, keys, nBinned, cells,
+                                   large, largeLo, largeHi, largeKeys, largeCells, dt, counts, offsets, 0, 0, cnt,
+                                   recorded, laneCounts, st, S, 0x7FFFu);
+    else
+        bp_large_large<BP_EMIT_RECORDED>((blockIdx.x - entryBlocks) * blockDim.x + threadIdx.x, F, large, largeSphere,
+                                         items, nItems, llCounts, llOffsets, 0, 0, cnt, st, chunkLo, chunkHi,
+                                         llRecorded, S);
 }
 
 // Pairs a caller injects in place of the broadphase (broadphaseExternalPairs,
@@ -2170,12 +2197,9 @@ __global__ void k_joint_flow(DevForces F)
 }
 
 // Joint::initialize (joint.cpp:35-54)
-__global__ void k_joint_init(DevBodies B, DevForces F, Params P, unsigned char *keep, const StepState *st = nullptr,
-                             int *orphanFlag = nullptr)
+AVBD_DEV void joint_initialize(const DevBodies &B, const DevForces &F, const Params &P, int j, unsigned char *keep,
+                               int *orphanFlag)
 {
-    int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= F.nJoint || step_aborted(st))
-        return;
     float4 *d = F.joint + 8 * (size_t)j;
     int2 ab = F.jointAB[j];
     float4 d0 = d[0], d1 = d[1], d3 = d[3], d4 = d[4], d5 = d[5], d6 = d[6], d7 = d[7];
@@ -2201,9 +2225,17 @@ __global__ void k_joint_init(DevBodies B, DevForces F, Params P, unsigned char *
     d[7] = f4(lamAng, 0.0f);
     if (F.jointFlow)
         joint_flow_start(F.jointFlow + 4 * (size_t)j, d);
-    keep[j] = d4.w != 0.0f ? 0 : 1;
+    if (keep)
+        keep[j] = d4.w != 0.0f ? 0 : 1;
     if (orphanFlag && (ab.x < 0 || B.massMoment[ab.x].x <= 0) && B.massMoment[ab.y].x <= 0)
         *orphanFlag = 1;
+}
+
+__global__ void k_joint_init(DevBodies B, DevForces F, Params P, unsigned char *keep, int *orphanFlag = nullptr)
+{
+    int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j < F.nJoint)
+        joint_initialize(B, F, P, j, keep, orphanFlag);
 }
 
 // Stable compaction of manifolds into the other buffer. With a device step state the count
@@ -2216,16 +2248,13 @@ constexpr int COMPACT_LANES = 8;
 // buffer the step started from and stays the live one.
 // `contactFlow`: the kept contacts' stamped words before the first iteration go there too
 // (avbd_iterate_flow.cuh; null: that kernel does not run).
-__global__ void k_manifold_compact(DevManifolds src, DevManifolds dst, int count, const unsigned char *keep,
-                                   const int *newIndex, StepState *st = nullptr, bool flip = true,
-                                   float4 *contactFlow = nullptr)
+AVBD_DEV void manifold_compact(long long t, const DevManifolds &src, const DevManifolds &dst, int count,
+                               const unsigned char *keep, const int *newIndex, StepState *st, bool flip,
+                               float4 *contactFlow)
 {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int m = (int)(t / COMPACT_LANES), lane = (int)(t % COMPACT_LANES);
     if (st)
     {
-        if (step_aborted(st))
-            return;
         count = st->nManBp;
         if (t == 0)
         {
@@ -2258,6 +2287,30 @@ __global__ void k_manifold_compact(DevManifolds src, DevManifolds dst, int count
         if (cf && (k & 3) == 3)
             cf[2 * (k >> 2) + 1] = make_float4(v.x, v.y, v.z, __uint_as_float(__float_as_uint(v.w) >> 31));
     }
+}
+
+__global__ void k_manifold_compact(DevManifolds src, DevManifolds dst, int count, const unsigned char *keep,
+                                   const int *newIndex, float4 *contactFlow = nullptr)
+{
+    manifold_compact((long long)blockIdx.x * blockDim.x + threadIdx.x, src, dst, count, keep, newIndex, nullptr, true,
+                     contactFlow);
+}
+
+// A device step's compaction, and after its blocks the joints' initialisation (which, like
+// it, may change the world only past the step's stop points).
+__global__ void k_forces_commit(DevManifolds src, DevManifolds dst, int capacity, const unsigned char *keep,
+                                const int *newIndex, StepState *st, float4 *contactFlow, DevBodies B, DevForces F,
+                                Params P, int *orphanFlag)
+{
+    if (step_aborted(st))
+        return;
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long compactThreads =
+        ((long long)capacity * COMPACT_LANES + blockDim.x - 1) / blockDim.x * blockDim.x;
+    if (t < compactThreads)
+        manifold_compact(t, src, dst, capacity, keep, newIndex, st, false, contactFlow);
+    else if (t - compactThreads < F.nJoint)
+        joint_initialize(B, F, P, (int)(t - compactThreads), nullptr, orphanFlag);
 }
 
 __global__ void k_joint_compact(int count, const unsigned char *keep, const int *newIndex, const int2 *abS,
@@ -2475,37 +2528,83 @@ __global__ void k_incidences_ranked(DevForces F, int n, unsigned *keys, unsigned
     vals[2 * rank + 1] = make_adj(type, 0u, (unsigned)idx);
 }
 
-// Segment starts of a sorted key array whose top bits are the segment id (0..n-1, or
-// larger for "no segment"); start[s] for s in [0, n] with gaps filled.
-template <class Key>
-__global__ void k_segment_starts(const Key *keys, int total, int shift, int n, int *start,
-                                 const StepState *st = nullptr)
+// Exclusive scan by one block of SCAN_BLOCK threads, tiles of four values a thread, the next
+// tile's read issued before the current one is added up. For lists of a few ten thousand
+// values: one launch of 3 to 6 us where the library scan is two, and the list's consumer or
+// the commit can follow in the same launch. load(i) for i < n, store(i, sum of the values
+// before i); returns the total to every thread.
+constexpr int SCAN_BLOCK = 1024, SCAN_SMALL = 32768;
+
+template <class Load, class Store>
+AVBD_DEV int block_scan(int n, Load load, Store store)
 {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= total || step_aborted(st))
-        return;
-    long long cur = (long long)(keys[k] >> shift);
-    if (cur > n)
-        cur = n;
-    long long prev = -1;
-    if (k > 0)
+    __shared__ int warpSum[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int carry = 0;
+    int v[4], next[4];
+    auto read = [&](int base, int(&x)[4]) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+        {
+            const int i = base + 4 * (int)threadIdx.x + u;
+            x[u] = i < n ? load(i) : 0;
+        }
+    };
+    read(0, v);
+    for (int base = 0; base < n; base += 4 * SCAN_BLOCK)
     {
-        prev = (long long)(keys[k - 1] >> shift);
-        if (prev > n)
-            prev = n;
+        if (base + 4 * SCAN_BLOCK < n)
+            read(base + 4 * SCAN_BLOCK, next);
+        const int mine = v[0] + v[1] + v[2] + v[3];
+        int incl = mine;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1)
+        {
+            const int o = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+            if (lane >= d)
+                incl += o;
+        }
+        if (lane == 31)
+            warpSum[warp] = incl;
+        __syncthreads();
+        int before = lane < warp ? warpSum[lane] : 0, all = warpSum[lane];
+        before = __reduce_add_sync(0xFFFFFFFFu, before);
+        all = __reduce_add_sync(0xFFFFFFFFu, all);
+        int at = carry + before + incl - mine;
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+        {
+            const int i = base + 4 * (int)threadIdx.x + u;
+            if (i < n)
+                store(i, at);
+            at += v[u];
+            v[u] = next[u];
+        }
+        carry += all;
+        __syncthreads(); // warpSum is read before the next tile writes it
     }
-    for (long long s = prev + 1; s <= cur; ++s)
-        start[s] = k;
-    if (k == total - 1)
-        for (long long s = cur + 1; s <= n; ++s)
-            start[s] = total;
+    return carry;
 }
 
-__global__ void k_copy_adj(const unsigned *vals, unsigned *adj, int total, const StepState *st = nullptr)
+// Which manifolds stay: their places (a device step's compaction).
+__global__ void __launch_bounds__(SCAN_BLOCK) k_keep_scan(const unsigned char *keep, int *index, int count,
+                                                          const StepState *st)
 {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < total && !step_aborted(st))
-        adj[k] = vals[k];
+    if (step_aborted(st))
+        return;
+    block_scan(min(count, st->nManBp), [&](int i) { return (int)keep[i]; }, [&](int i, int at) { index[i] = at; });
+}
+
+// First rows of the force-list entries (`count` entries and the end; with a device step state
+// the live ones).
+__global__ void __launch_bounds__(SCAN_BLOCK) k_row_scan(const int *rows, int *first, int count, int otherForces,
+                                                         const StepState *st)
+{
+    if (step_aborted(st))
+        return;
+    if (st)
+        count = min(count, 2 * (st->nMan + otherForces));
+    block_scan(count + 1, [&](int i) { return i < count ? rows[i] : 0; }, [&](int i, int at) { first[i] = at; });
 }
 
 // ---------------------------------------------------------------------------
@@ -2522,11 +2621,51 @@ AVBD_DEV bool finite4(float4 v) { return isfinite(v.x) && isfinite(v.y) && isfin
 // path) collects STEP_SEEN_* bits for the host.
 constexpr int STEP_SEEN_NONFINITE = 1, STEP_SEEN_BROKEN_JOINT = 2;
 
-__global__ void k_step_begin(DevBodies B, const float4 *joint, int nJoint, StepState *st, int *seen)
+// What a step starts from cleared: counters, hash tables, control blocks (each a whole number
+// of 4-byte words, 16-byte aligned) and the worlds' bounds, all in the step's first launch
+// instead of a memset or a kernel each in the chain of small launches.
+struct StepClear
 {
+    static constexpr int MAX = 10;
+    unsigned *p[MAX];
+    long long words[MAX];
+    unsigned value[MAX];
+    int count = 0;
+    unsigned *bounds = nullptr; // eight words per world
+    int worlds = 0;
+    uint4 *chunkLo = nullptr; // lower bounds of the large-list chunks
+    int chunks = 0;
+    long long most = 0; // words of the largest region
+
+    void add(void *region, size_t bytes, unsigned v)
+    {
+        p[count] = (unsigned *)region;
+        words[count] = (long long)(bytes / 4);
+        value[count] = v;
+        most = words[count] > most ? words[count] : most;
+        ++count;
+    }
+};
+
+__global__ void k_step_begin(DevBodies B, const float4 *joint, int nJoint, StepState *st, int *seen, StepClear C)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    for (int r = 0; r < C.count; ++r)
+    {
+        const unsigned v = C.value[r];
+        const long long quads = C.words[r] / 4;
+        for (long long k = t; k < quads; k += stride)
+            ((uint4 *)C.p[r])[k] = make_uint4(v, v, v, v);
+        if (t < C.words[r] - 4 * quads)
+            C.p[r][4 * quads + t] = v;
+    }
+    for (long long k = t; k < 8ll * C.worlds; k += stride) // mins, then maxima and the largest binned slack
+        C.bounds[k] = (k & 7) < 3 ? 0xFFFFFFFFu : 0u;
+    for (long long k = t; k < C.chunks; k += stride)
+        C.chunkLo[k] = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u);
     if (step_aborted(st))
         return;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
     bool bad = false, broke = false;
     if (t < B.n)
         bad = !finite4(B.pos[t]) || !finite4(B.quat[t]) || !finite4(B.vel[t]) || !finite4(B.angvel[t]);
@@ -3136,33 +3275,40 @@ AVBD_DEV int rows_listed(const DevForces &F, unsigned e)
     }
 }
 
-// Row list, built in parallel over the force-list entries (sorted incidence keys carry the
-// body): entry k contributes rows_listed rows unless its body is static (never solved).
-// Incidences without a body (the world side of an anchored joint) sort after the last body
-// and contribute none.
+// From the sorted incidences (keys: body << shift | order, n or above for none), everything
+// that one pass over them gives: the bodies' force lists (start for each body 0 .. n, gaps
+// filled, and entries) and each entry's number of constraint rows. Entry k contributes
+// rows_listed rows unless its body is static (never solved). Incidences without a body (the
+// world side of an anchored joint) sort after the last body and contribute none.
 template <class Key>
-__global__ void k_entry_rows(DevForces F, DevBodies B, const Key *sortedKeys, int total, int shift,
-                             int *count, const StepState *st = nullptr)
+__global__ void k_force_lists(DevForces F, DevBodies B, const Key *keys, const unsigned *vals, int total, int shift,
+                              int *start, unsigned *adj, int *rowCount, const StepState *st = nullptr)
 {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k > total || step_aborted(st))
         return;
-    int r = 0;
-    if (k < total)
+    if (k == total)
     {
-        unsigned long long b = sortedKeys[k] >> shift;
-        if (b < (unsigned long long)B.n && B.massMoment[b].x > 0)
-            r = rows_listed(F, F.adj[k]);
+        rowCount[k] = 0; // so the exclusive scan ends with the row total
+        return;
     }
-    count[k] = r; // count[total] = 0, so the exclusive scan ends with the row total
-}
-
-__global__ void k_row_starts(const int *adjStart, const int *entryRow, int n, int *rowStart,
-                             const StepState *st = nullptr)
-{
-    int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b <= n && !step_aborted(st))
-        rowStart[b] = entryRow[adjStart[b]];
+    const long long n = B.n;
+    const unsigned long long body = (unsigned long long)keys[k] >> shift;
+    const unsigned e = vals[k];
+    adj[k] = e;
+    rowCount[k] = body < (unsigned long long)n && B.massMoment[body].x > 0 ? rows_listed(F, e) : 0;
+    const long long cur = body > (unsigned long long)n ? n : (long long)body;
+    long long prev = -1;
+    if (k > 0)
+    {
+        const unsigned long long p = (unsigned long long)keys[k - 1] >> shift;
+        prev = p > (unsigned long long)n ? n : (long long)p;
+    }
+    for (long long s = prev + 1; s <= cur; ++s)
+        start[s] = k;
+    if (k == total - 1)
+        for (long long s = cur + 1; s <= n; ++s)
+            start[s] = total;
 }
 
 // The other body of a force-list entry (-1: the world side of an anchored joint).
@@ -3199,11 +3345,16 @@ constexpr int ROW_PARTNER_LATER = (int)0x80000000u;
 AVBD_DEV int row_sub(int2 row) { return row.y & 7; }
 AVBD_DEV int row_partner(int2 row) { return ((row.y & (ROW_OWNS_DUAL - 1)) >> 3) - 1; }
 
-__global__ void k_entry_fill(DevForces F, const int *entryRow, const int *count, int total,
+// The row list and each body's range in it.
+__global__ void k_entry_fill(DevForces F, const int *entryRow, const int *count, int total, int bodies, int *rowStart,
                              const StepState *st = nullptr)
 {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= total || step_aborted(st))
+    if (step_aborted(st))
+        return;
+    if (k <= bodies)
+        rowStart[k] = entryRow[F.adjStart[k]];
+    if (k >= total)
         return;
     int out = entryRow[k];
     unsigned e = F.adj[k];
