@@ -3965,16 +3965,16 @@ __global__ void __launch_bounds__(BLOCK, 1) k_iterations(DevBodies B, DevForces 
 // Greedy colouring in list order as one dataflow pass (the default colouring mode)
 // ---------------------------------------------------------------------------
 
-AVBD_DEV unsigned long long ld_acquire_u64(const unsigned long long *p)
+AVBD_DEV unsigned long long ld_relaxed_u64(const unsigned long long *p)
 {
     unsigned long long v;
-    asm volatile("ld.acquire.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
 
-AVBD_DEV void st_release_u64(unsigned long long *p, unsigned long long v)
+AVBD_DEV void st_relaxed_u64(unsigned long long *p, unsigned long long v)
 {
-    asm volatile("st.release.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
 // With list-index priority the Jones-Plassmann rounds colour a vertex once every
@@ -3985,7 +3985,16 @@ AVBD_DEV void st_release_u64(unsigned long long *p, unsigned long long v)
 // finished every smaller vertex of its grid-stride sequence and all blocks are resident),
 // so the waits cannot cycle; each is bounded and on expiry records ctl->error and gives up.
 // `state` holds (epoch << 32 | round << 16 | colour) of the vertices coloured in the launch
-// with that epoch, so nothing needs clearing between launches.
+// with that epoch, so nothing needs clearing between launches. Such a word is all that passes
+// between warps before the grid barrier, so it is written and read relaxed: no fence, and no
+// acquire to empty L1 on every poll.
+//
+// A vertex with one lower neighbour takes colour 0, or 1 if that neighbour has 0. Down a chain
+// of such vertices (a jointed chain) the colours alternate from its first vertex's, so a
+// warp finds for each of them the lane its chain starts from and the distance (pointer
+// doubling, five shuffles) and colours all of them in the pass after that lane, instead of a
+// link a pass. Measured: 64 uneven worlds with jointed chains up to 1,168 links 304 -> 65 us, 512
+// worlds (up to 2,026 links) 583 -> 126, 262,144 boxes in stacks 82 -> 77.
 //
 // The same cooperative launch then places the vertices in colour order, ascending body
 // index inside each colour (what sorting (colour, body) keys gives): block b counts the
@@ -4044,17 +4053,37 @@ __global__ void __launch_bounds__(COLOUR_FLOW_BLOCK) k_colour_greedy(
                     // static bodies are not vertices; a dynamic neighbour shares this force
                     if (u < 0 || u >= v || B.massMoment[u].x <= 0)
                         continue;
+                    bool known = false; // another force of the same two bodies
+#pragma unroll
+                    for (int j = 0; j < NB; ++j)
+                        known = known || (j < nnb && nb[j] == u);
+                    if (known)
+                        continue;
                     if (nnb < NB)
                     {
                         if (u >= base)
                             intra |= 1u << nnb;
-                        nb[nnb++] = u;
+#pragma unroll
+                        for (int j = 0; j < NB; ++j)
+                            nb[j] = j == nnb ? u : nb[j];
+                        ++nnb;
                     }
                     else
                         many = true;
                 }
         }
         const unsigned all = (1u << nnb) - 1u;
+        // one lower neighbour, a lane of this warp: `from` the lane its chain starts from
+        const bool link = pending && !many && nnb == 1 && intra != 0u;
+        int from = link ? nb[0] - base : lane, links = link ? 1 : 0;
+#pragma unroll
+        for (int d = 0; d < 5; ++d)
+        {
+            links += __shfl_sync(0xFFFFFFFFu, links, from);
+            from = __shfl_sync(0xFFFFFFFFu, from, from);
+        }
+        if (link)
+            intra = 0u;
         // shuffle passes look at the first kIntra neighbours (the warp's largest in-warp one)
         const int kIntra = __reduce_max_sync(0xFFFFFFFFu, 32 - __clz((int)intra));
         // takes the smallest colour no lower neighbour uses; `state` is written at the end of
@@ -4086,9 +4115,9 @@ __global__ void __launch_bounds__(COLOUR_FLOW_BLOCK) k_colour_greedy(
 #pragma unroll
                 for (int k = 0; k < NB; ++k)
                 {
-                    if (k >= nnb || (((seen | intra) >> k) & 1u))
+                    if (link || k >= nnb || (((seen | intra) >> k) & 1u))
                         continue;
-                    const unsigned long long su = ld_acquire_u64(&state[nb[k]]);
+                    const unsigned long long su = ld_relaxed_u64(&state[nb[k]]);
                     if ((su >> 32) != (unsigned long long)epoch)
                         continue;
                     const int cu = (int)(su & 0xFFFFu), ru = (int)((su >> 16) & 0xFFFFu);
@@ -4113,7 +4142,7 @@ __global__ void __launch_bounds__(COLOUR_FLOW_BLOCK) k_colour_greedy(
                     int u = ab.x == v ? ab.y : ab.x;
                     if (u < 0 || u >= v || B.massMoment[u].x <= 0)
                         continue;
-                    const unsigned long long su = ld_acquire_u64(&state[u]);
+                    const unsigned long long su = ld_relaxed_u64(&state[u]);
                     if ((su >> 32) != (unsigned long long)epoch)
                     {
                         ready = false;
@@ -4150,8 +4179,19 @@ __global__ void __launch_bounds__(COLOUR_FLOW_BLOCK) k_colour_greedy(
                         seen |= 1u << k;
                     }
                 }
-                if (pending && !many && seen == all)
+                if (pending && !many && !link && seen == all)
                 {
+                    take();
+                    took = true;
+                    progressed = true;
+                }
+                const unsigned start = __shfl_sync(0xFFFFFFFFu, mine_cr, from);
+                if (pending && link && start != ~0u)
+                {
+                    // the neighbour's colour is 0: this vertex takes 1, else 0
+                    const bool startsAt0 = (start & 0xFFFFu) == 0u, odd = (links & 1) != 0;
+                    used[0] = startsAt0 == odd ? 1ull : 0ull;
+                    round = (int)(start >> 16) + links;
                     take();
                     took = true;
                     progressed = true;
@@ -4161,7 +4201,7 @@ __global__ void __launch_bounds__(COLOUR_FLOW_BLOCK) k_colour_greedy(
             }
             if (publish)
             {
-                st_release_u64(&state[v], ((unsigned long long)epoch << 32) | (unsigned long long)mine_cr);
+                st_relaxed_u64(&state[v], ((unsigned long long)epoch << 32) | (unsigned long long)mine_cr);
                 publish = false;
             }
             if (__any_sync(0xFFFFFFFFu, progressed))
