@@ -57,10 +57,8 @@ struct StepTape
     const int *src;      // per slot: slot of the previous step's list, -1 = new contact
     const unsigned char *iflags;
     const int *pairIdx; // per manifold: friction pair
-    const int *adjStart;
-    const unsigned *adj;
-    const int *solveList;
-    const int *colour;
+    const int4 *entries; // solved bodies in colour order: body, first row, end of its rows
+    const int2 *rows;    // contact rows in force order, with the partner and its colour's place
     const unsigned char *bflags;
     const unsigned short *flags; // iterations x 8 nMan
 };
@@ -560,6 +558,7 @@ template <int G> AVBD_DEV D group_sum(D v, unsigned mask)
     return v;
 }
 
+// The factorisation reads the lower triangle alone.
 template <int G> AVBD_DEV void group_sum_sys(ad::Sys6<D> &s, unsigned mask)
 {
 #pragma unroll
@@ -567,14 +566,37 @@ template <int G> AVBD_DEV void group_sum_sys(ad::Sys6<D> &s, unsigned mask)
     {
         s.g[i] = group_sum<G>(s.g[i], mask);
 #pragma unroll
-        for (int j = 0; j < 6; ++j)
+        for (int j = 0; j <= i; ++j)
             s.H[i][j] = group_sum<G>(s.H[i][j], mask);
     }
 }
 
-// body primal for the bodies of one colour (solver.cpp:1177-1242)
+// One contact row of a body (a listed row of the taped step).
+struct AdjRow
+{
+    int m, ci, slot, partner;
+    bool isA, partnerMoved; // partnerMoved: it has an earlier colour, so it moved in this iteration
+};
+
+AVBD_DEV AdjRow adj_row(int2 row)
+{
+    AdjRow r;
+    r.m = (int)adj_index((unsigned)row.x);
+    r.ci = row_sub(row);
+    r.slot = 8 * r.m + r.ci;
+    r.partner = row_partner(row);
+    r.isA = adj_isA((unsigned)row.x) != 0;
+    r.partnerMoved = (row.y & ROW_OWNS_DUAL) == 0;
+    return r;
+}
+
+// body primal for the bodies of one colour (solver.cpp:1177-1242). Bound by the chain of
+// dependent loads and double-precision divisions, not by throughput (a colour of the
+// 1,000-box tower is 500 bodies): a lane reaches its rows through the taped row list, two
+// loads after the solve entry, where walking the body's force list took two per manifold.
+// poseNext: the snapshot slice after this iteration (null: no snapshots).
 __global__ void __launch_bounds__(ADJ_BLOCK) k_rep_primal(StepTape T, DevBodies B, State64 S, AdjParams Q, int t,
-                                                          int first, int count, double *ldlOut)
+                                                          int first, int count, double *ldlOut, double4 *poseNext)
 {
     constexpr int G = ADJ_G;
     const int lane = threadIdx.x % G;
@@ -582,35 +604,24 @@ __global__ void __launch_bounds__(ADJ_BLOCK) k_rep_primal(StepTape T, DevBodies 
     if (gid >= count)
         return;
     const unsigned mask = group_mask<G>();
-    const int b = T.solveList[first + gid];
+    const int4 ent = T.entries[first + gid];
+    const int b = ent.x;
     float4 mm = B.massMoment[b];
     ad::Pose<D> own = pose_state(S, b);
     const unsigned short *fl = T.flags + (size_t)t * 8 * T.nMan;
     ad::Sys6<D> sys;
     ad::sys_zero(sys);
-    int row = 0;
-    for (int k = T.adjStart[b]; k < T.adjStart[b + 1]; ++k)
+    for (int k = ent.y + lane; k < ent.z; k += G)
     {
-        unsigned e = T.adj[k];
-        if (adj_type(e) != ADJ_MANIFOLD)
-            continue;
-        int m = (int)adj_index(e);
-        int nc = T.nc[m];
-        int mine = row % G <= lane ? lane - row % G : lane - row % G + G; // first owned contact
-        row += nc;
-        if (mine >= nc)
-            continue;
-        bool isA = adj_isA(e) != 0;
-        int2 ab = T.ab[m];
-        ad::Pose<D> A = isA ? own : pose_state(S, ab.x);
-        ad::Pose<D> Bp = isA ? pose_state(S, ab.y) : own;
-        for (int ci = mine; ci < nc; ci += G)
-        {
-            int s = m * 8 + ci;
-            ad::ContactIn<D> c = contact64(T, m, ci, ld3(S.c0 + s), ld3(S.lam + s), ld3(S.pen + s));
-            ad::stamp_contact(sys, c, ad::contact_forward(A, Bp, c, Q.alpha, primal_bits(fl[s], isA)), isA);
-        }
+        const AdjRow r = adj_row(T.rows[k]);
+        const ad::Pose<D> other = pose_state(S, r.partner);
+        ad::ContactIn<D> c = contact64(T, r.m, r.ci, ld3(S.c0 + r.slot), ld3(S.lam + r.slot), ld3(S.pen + r.slot));
+        ad::stamp_contact(sys, c,
+                          ad::contact_forward(r.isA ? own : other, r.isA ? other : own, c, Q.alpha,
+                                              primal_bits(fl[r.slot], r.isA)),
+                          r.isA);
     }
+    __syncwarp(mask);
     group_sum_sys<G>(sys, mask);
     ad::stamp_inertia(sys, (D)mm.x, shape_of(mm), own.p, ld3(S.tLin + b), own.q, ld4(S.tAng + b), Q.dt);
     ad::Ldl6<D> f;
@@ -619,15 +630,22 @@ __global__ void __launch_bounds__(ADJ_BLOCK) k_rep_primal(StepTape T, DevBodies 
     ad::body_dx(f, sys, dx);
     if (lane == 0)
     {
-        st3(S.p + b, own.p + ad::v3<D>(dx[0], dx[1], dx[2]));
-        st4(S.q + b, ad::qstep(own.q, ad::v3<D>(dx[3], dx[4], dx[5])));
+        const ad::V3<D> p = own.p + ad::v3<D>(dx[0], dx[1], dx[2]);
+        const ad::Q4<D> q = ad::qstep(own.q, ad::v3<D>(dx[3], dx[4], dx[5]));
+        st3(S.p + b, p);
+        st4(S.q + b, q);
+        if (poseNext)
+        {
+            st3(poseNext + b, p);
+            st4(poseNext + T.n + b, q);
+        }
         if (ldlOut)
             store_ldl(ldlOut + ((size_t)t * T.n + b) * LDL_STRIDE, f, dx);
     }
 }
 
-// Manifold::updateDual (manifold.cpp:231-279)
-__global__ void k_rep_dual(StepTape T, State64 S, AdjParams Q, int t)
+// Manifold::updateDual (manifold.cpp:231-279); lpNext: the snapshot slice after this iteration
+__global__ void k_rep_dual(StepTape T, State64 S, AdjParams Q, int t, double4 *lpNext)
 {
     int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= 8 * T.nMan)
@@ -642,6 +660,11 @@ __global__ void k_rep_dual(StepTape T, State64 S, AdjParams Q, int t)
                              dual_bits(T.flags[(size_t)t * 8 * T.nMan + s]), lam, pen);
     st3(S.lam + s, lam);
     st3(S.pen + s, pen);
+    if (lpNext)
+    {
+        st3(lpNext + s, lam);
+        st3(lpNext + 8 * (size_t)T.nMan + s, pen);
+    }
 }
 
 // finishStep (solver.cpp:1275-1287)
@@ -659,20 +682,30 @@ __global__ void k_rep_finish(StepTape T, DevBodies B, State64 S, AdjParams Q)
     st3(S.w + b, ad::qdiff(ld4(S.q + b), ld4(S.iAng + b)) * idt);
 }
 
-// replay state at an iteration boundary: poses of every body, lambda and penalty of every slot
-__global__ void k_snapshot(State64 S, int n, int nMan, double4 *pose, double4 *lp)
+// Every slice of a step's snapshots (poses of every body, lambda and penalty of every slot, at
+// each iteration boundary) as the replay state before the first iteration; the primal and
+// the dual then write what they change into the slice after their iteration.
+__global__ void k_snapshot_fill(State64 S, int n, int nMan, double4 *pose, double4 *lp, int slices)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const size_t slots = 8 * (size_t)nMan;
     if (i < n)
     {
-        pose[i] = S.p[i];
-        pose[n + i] = S.q[i];
+        const double4 p = S.p[i], q = S.q[i];
+        for (int t = 0; t < slices; ++t)
+        {
+            pose[(size_t)t * 2 * n + i] = p;
+            pose[(size_t)t * 2 * n + n + i] = q;
+        }
     }
-    int slots = 8 * nMan;
-    if (i < slots)
+    if (i < (int)slots)
     {
-        lp[i] = S.lam[i];
-        lp[slots + i] = S.pen[i];
+        const double4 l = S.lam[i], k = S.pen[i];
+        for (int t = 0; t < slices; ++t)
+        {
+            lp[(size_t)t * 2 * slots + i] = l;
+            lp[(size_t)t * 2 * slots + slots + i] = k;
+        }
     }
 }
 
@@ -779,7 +812,7 @@ __global__ void k_adj_dual(StepTape T, Snap64 X, DevBodies B, AdjView A, AdjPara
 
 // body primal of iteration t for the bodies of colour c, lanes as in k_rep_primal
 __global__ void __launch_bounds__(ADJ_BLOCK) k_adj_primal(StepTape T, Snap64 X, DevBodies B, AdjView A, AdjParams Q,
-                                                          int t, int c, int first, int count)
+                                                          int t, int first, int count)
 {
     constexpr int G = ADJ_G;
     const int lane = threadIdx.x % G;
@@ -788,14 +821,10 @@ __global__ void __launch_bounds__(ADJ_BLOCK) k_adj_primal(StepTape T, Snap64 X, 
         return;
     const unsigned mask = group_mask<G>();
     const int n = T.n;
-    const int b = T.solveList[first + gid];
-    auto partner = [&](int x) {
-        int cx = T.colour[x];
-        return pose_snap(X, n, (cx >= 0 && cx < c) ? t + 1 : t, x);
-    };
+    const int4 ent = T.entries[first + gid];
+    const int b = ent.x;
     const unsigned short *fl = T.flags + (size_t)t * 8 * T.nMan;
     ad::Pose<D> own = pose_snap(X, n, t, b);
-    const int start = T.adjStart[b], end = T.adjStart[b + 1];
     float4 mm = B.massMoment[b];
     D mass = mm.x;
     ad::V3<D> shape = shape_of(mm);
@@ -818,52 +847,30 @@ __global__ void __launch_bounds__(ADJ_BLOCK) k_adj_primal(StepTape T, Snap64 X, 
     ad::body_dx_vjp_u(f, dxbar, u);
     // each lane's rows
     ad::PoseBar<D> mineBar = ad::posebar_zero<D>();
+    for (int k = ent.y + lane; k < ent.z; k += G)
     {
-        int row = 0;
-        for (int k = start; k < end; ++k)
-        {
-            unsigned e = T.adj[k];
-            if (adj_type(e) != ADJ_MANIFOLD)
-                continue;
-            int m = (int)adj_index(e);
-            int nc = T.nc[m];
-            int mine = row % G <= lane ? lane - row % G : lane - row % G + G;
-            row += nc;
-            if (mine >= nc)
-                continue;
-            bool isA = adj_isA(e) != 0;
-            int2 ab = T.ab[m];
-            ad::Pose<D> PA = isA ? own : partner(ab.x);
-            ad::Pose<D> PB = isA ? partner(ab.y) : own;
-            ad::PoseBar<D> Ob = ad::posebar_zero<D>();
-            D mub = 0;
-            for (int ci = mine; ci < nc; ci += G)
-            {
-                int s = m * 8 + ci;
-                ad::ContactIn<D> cc = contact_snap(T, X, t, m, ci);
-                ad::PoseBar<D> Ab = ad::posebar_zero<D>(), Bb = ad::posebar_zero<D>();
-                ad::V3<D> lb = ld3(A.lam + s), pnb = ld3(A.pen + s), c0b = ld3(A.c0 + s);
-                ad::contact_primal_vjp_outer(PA, PB, cc, Q.alpha, primal_bits(fl[s], isA), isA, u, dx, Ab, Bb, lb,
-                                             pnb, c0b, mub);
-                st3(A.lam + s, lb);
-                st3(A.pen + s, pnb);
-                st3(A.c0 + s, c0b);
-                const ad::PoseBar<D> &me = isA ? Ab : Bb;
-                const ad::PoseBar<D> &them = isA ? Bb : Ab;
-                mineBar.p += me.p;
-                mineBar.q += me.q;
-                mineBar.pi += me.pi;
-                mineBar.qi += me.qi;
-                Ob.p += them.p;
-                Ob.q += them.q;
-                Ob.pi += them.pi;
-                Ob.qi += them.qi;
-            }
-            scatter_pose(B, A, isA ? ab.y : ab.x, Ob);
-            if (mub != 0 && T.pairIdx[m] >= 0)
-                atomicAdd(A.mu + T.pairIdx[m], mub);
-        }
+        const AdjRow r = adj_row(T.rows[k]);
+        const int s = r.slot;
+        const ad::Pose<D> other = pose_snap(X, n, r.partnerMoved ? t + 1 : t, r.partner);
+        ad::ContactIn<D> cc = contact_snap(T, X, t, r.m, r.ci);
+        ad::PoseBar<D> Ab = ad::posebar_zero<D>(), Bb = ad::posebar_zero<D>();
+        ad::V3<D> lb = ld3(A.lam + s), pnb = ld3(A.pen + s), c0b = ld3(A.c0 + s);
+        D mub = 0;
+        ad::contact_primal_vjp_outer(r.isA ? own : other, r.isA ? other : own, cc, Q.alpha,
+                                     primal_bits(fl[s], r.isA), r.isA, u, dx, Ab, Bb, lb, pnb, c0b, mub);
+        st3(A.lam + s, lb);
+        st3(A.pen + s, pnb);
+        st3(A.c0 + s, c0b);
+        const ad::PoseBar<D> &me = r.isA ? Ab : Bb;
+        mineBar.p += me.p;
+        mineBar.q += me.q;
+        mineBar.pi += me.pi;
+        mineBar.qi += me.qi;
+        scatter_pose(B, A, r.partner, r.isA ? Bb : Ab);
+        if (mub != 0 && T.pairIdx[r.m] >= 0)
+            atomicAdd(A.mu + T.pairIdx[r.m], mub);
     }
+    __syncwarp(mask);
     // the body's own share, summed over the group
     D r[14] = {mineBar.p.x, mineBar.p.y, mineBar.p.z, mineBar.q.x, mineBar.q.y, mineBar.q.z, mineBar.q.w,
                mineBar.pi.x, mineBar.pi.y, mineBar.pi.z, mineBar.qi.x, mineBar.qi.y, mineBar.qi.z, mineBar.qi.w};
@@ -976,9 +983,8 @@ struct TapeStep
     DArr<int> src;
     DArr<unsigned char> iflags;
     DArr<int> pairIdx;
-    DArr<int> adjStart;
-    DArr<unsigned> adj;
-    DArr<int> solveList, colour;
+    DArr<int4> entries;
+    DArr<int2> rows;
     DArr<unsigned char> bflags;
     DArr<unsigned short> flags;
 };
@@ -1023,6 +1029,7 @@ struct AdjointState
     int rcur = 0;
     size_t rCap = 0;
     std::vector<SegSnap> snap; // two sets of `every` steps: replay of one segment, reverse of another
+    bool lastKept = false;     // the last segment's set still holds the forward's snapshots
     // The double-precision replay runs on its own stream, overlapping the FP32 steps (forward)
     // and the reverse sweep of the next segment (backward); events order the two.
     cudaStream_t side = nullptr;
@@ -1101,10 +1108,8 @@ void release_tape(TapeStep &s)
     release(s.src);
     release(s.iflags);
     release(s.pairIdx);
-    release(s.adjStart);
-    release(s.adj);
-    release(s.solveList);
-    release(s.colour);
+    release(s.entries);
+    release(s.rows);
     release(s.bflags);
     release(s.flags);
 }
@@ -1214,20 +1219,16 @@ int rec_prepared(AvbdContext *ctx)
                                                                       s.src.p, s.iflags.p);
         LAUNCHED();
     }
-    // force lists of this step (n + 1 starts; the entry count is the last start)
-    CHECK(reserve(ctx, s.adjStart, (size_t)n + 1, false));
-    CHECK(copy_d2d(ctx, s.adjStart.p, ctx->adjStart.p, (size_t)n + 1));
-    CU(cudaMemcpyAsync(ctx->hScalars + 2, ctx->adjStart.p + n, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    // the solved bodies with their row ranges, and the rows (their count is the last start)
+    CU(cudaMemcpyAsync(ctx->hScalars + 2, ctx->rowStart.p + n, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     CU(cudaStreamSynchronize(ctx->stream));
-    int nAdj = 0;
-    std::memcpy(&nAdj, ctx->hScalars + 2, sizeof(int));
-    CHECK(reserve(ctx, s.adj, (size_t)std::max(nAdj, 1), false));
-    CHECK(copy_d2d(ctx, s.adj.p, ctx->adj.p, (size_t)nAdj));
+    int nRows = 0;
+    std::memcpy(&nRows, ctx->hScalars + 2, sizeof(int));
+    CHECK(reserve(ctx, s.rows, (size_t)std::max(nRows, 1), false));
+    CHECK(copy_d2d(ctx, s.rows.p, ctx->rows.p, (size_t)nRows));
     s.nSolve = ctx->nSolve;
-    CHECK(reserve(ctx, s.solveList, (size_t)std::max(ctx->nSolve, 1), false));
-    CHECK(copy_d2d(ctx, s.solveList.p, ctx->solveList.p, (size_t)ctx->nSolve));
-    CHECK(reserve(ctx, s.colour, (size_t)std::max(n, 1), false));
-    CHECK(copy_d2d(ctx, s.colour.p, ctx->colour.p, (size_t)n));
+    CHECK(reserve(ctx, s.entries, (size_t)std::max(ctx->nSolve, 1), false));
+    CHECK(copy_d2d(ctx, s.entries.p, ctx->solveEntry.p, (size_t)ctx->nSolve));
     s.colourStart = ctx->hColourStart;
     CHECK(reserve(ctx, s.bflags, (size_t)std::max(n, 1), false));
     k_tape_bflags<<<grid_for(n, 256), 256, 0, ctx->stream>>>(dev_bodies(ctx), a->bodyIn32.p, ctx->adjStart.p,
@@ -1288,7 +1289,7 @@ int rec_finish(AvbdContext *ctx)
     X.basis = mb.basis.p;
     X.ab = mb.ab.p;
     X.nc = mb.n.p;
-    X.colour = s.colour.p;
+    X.colour = ctx->colour.p;
     long long total = 8ll * M * s.iterations;
     k_tape_flags<<<grid_for(total, 128), 128, 0, ctx->stream>>>(X, dev_params(ctx->params), s.iterations,
                                                                  s.flags.p);
@@ -1308,10 +1309,8 @@ StepTape tape_view(AvbdContext *ctx, const TapeStep &s)
     T.src = s.src.p;
     T.iflags = s.iflags.p;
     T.pairIdx = s.pairIdx.p;
-    T.adjStart = s.adjStart.p;
-    T.adj = s.adj.p;
-    T.solveList = s.solveList.p;
-    T.colour = s.colour.p;
+    T.entries = s.entries.p;
+    T.rows = s.rows.p;
     T.bflags = s.bflags.p;
     T.flags = s.flags.p;
     return T;
@@ -1368,6 +1367,27 @@ State64 state_view(AdjointState *a)
 
 int prev_man(AdjointState *a, int s) { return s > 0 ? a->tape[s - 1].nMan : a->nMan0; }
 
+// Snapshots of one step: bytes, and their buffers (reserved on the context stream while no
+// replay reads or writes them).
+constexpr size_t LAST_SEGMENT_BYTES = (size_t)1 << 30;
+
+size_t snap_bytes(int n, int M, int iterations)
+{
+    const size_t T1 = (size_t)iterations + 1;
+    return sizeof(double4) * (5 * (size_t)n + T1 * (2 * (size_t)n + 16 * (size_t)M) + 8 * (size_t)M) +
+           sizeof(double) * (size_t)iterations * n * LDL_STRIDE;
+}
+
+int snap_reserve(AvbdContext *ctx, SegSnap &snap, int n, int M, int iterations)
+{
+    const size_t T1 = (size_t)iterations + 1, n1 = (size_t)std::max(n, 1), m1 = (size_t)std::max(M, 1);
+    CHECK(reserve(ctx, snap.bodyIn, 5 * n1, false));
+    CHECK(reserve(ctx, snap.pose, T1 * 2 * n1, false));
+    CHECK(reserve(ctx, snap.lp, T1 * 16 * m1, false));
+    CHECK(reserve(ctx, snap.c0, 8 * m1, false));
+    return reserve(ctx, snap.ldl, (size_t)iterations * n1 * LDL_STRIDE, false);
+}
+
 // Replays taped step s on the replay stream; with `snap`, keeps what the reverse sweep reads.
 int replay_step(AvbdContext *ctx, int s, SegSnap *snap)
 {
@@ -1402,33 +1422,31 @@ int replay_step(AvbdContext *ctx, int s, SegSnap *snap)
     k_rep_warm<<<grid_for(n, 128), 128, 0, st>>>(T, B, S, Q);
     LAUNCHED();
     int C = (int)ts.colourStart.size() - 1;
-    auto snapshot = [&](int t) -> int {
-        if (!snap)
-            return AVBD_OK;
-        k_snapshot<<<grid_for(std::max<long long>(n, 8ll * M), 256), 256, 0, st>>>(
-            S, n, M, snap->pose.p + (size_t)t * 2 * n, snap->lp.p + (size_t)t * 16 * M);
+    if (snap)
+    {
+        k_snapshot_fill<<<grid_for(std::max<long long>(n, 8ll * M), 128), 128, 0, st>>>(S, n, M, snap->pose.p,
+                                                                                       snap->lp.p, (int)T1);
         LAUNCHED();
-        return AVBD_OK;
-    };
+    }
     for (int t = 0; t < ts.iterations; ++t)
     {
-        CHECK(snapshot(t));
         for (int c = 0; c < C; ++c)
         {
             int first = ts.colourStart[c], count = ts.colourStart[c + 1] - first;
             if (count <= 0)
                 continue;
             k_rep_primal<<<grid_for(count, ADJ_BLOCK / ADJ_G), ADJ_BLOCK, 0, st>>>(
-                T, B, S, Q, t, first, count, snap ? snap->ldl.p : nullptr);
+                T, B, S, Q, t, first, count, snap ? snap->ldl.p : nullptr,
+                snap ? snap->pose.p + (size_t)(t + 1) * 2 * n : nullptr);
             LAUNCHED();
         }
         if (M)
         {
-            k_rep_dual<<<grid_for(8ll * M, 128), 128, 0, st>>>(T, S, Q, t);
+            k_rep_dual<<<grid_for(8ll * M, 128), 128, 0, st>>>(T, S, Q, t,
+                                                              snap ? snap->lp.p + (size_t)(t + 1) * 16 * M : nullptr);
             LAUNCHED();
         }
     }
-    CHECK(snapshot(ts.iterations));
     k_rep_finish<<<grid_for(n, 128), 128, 0, st>>>(T, B, S, Q);
     LAUNCHED();
     a->rcur ^= 1;
@@ -1542,8 +1560,8 @@ int reverse_step(AvbdContext *ctx, int s, const SegSnap &snap)
             int first = ts.colourStart[c], count = ts.colourStart[c + 1] - first;
             if (count <= 0)
                 continue;
-            k_adj_primal<<<grid_for(count, ADJ_BLOCK / ADJ_G), ADJ_BLOCK, 0, ctx->stream>>>(T, X, B, A, Q, t, c,
-                                                                                              first, count);
+            k_adj_primal<<<grid_for(count, ADJ_BLOCK / ADJ_G), ADJ_BLOCK, 0, ctx->stream>>>(T, X, B, A, Q, t, first,
+                                                                                              count);
             LAUNCHED();
         }
     }
@@ -1638,6 +1656,13 @@ int avbd_adjoint_forward(AvbdContext *ctx, int32_t nsteps, int32_t checkpoint_ev
         LAUNCHED();
     }
     CHECK(side_after_main(ctx));
+    // The forward's replay of the last segment keeps its snapshots, which the backward starts
+    // with, where they are small (LAST_SEGMENT_BYTES: what a forward alone may hold for it).
+    const int lastSeg = nck - 1, lastStep = lastSeg * checkpoint_every;
+    if ((int)a->snap.size() < 2 * checkpoint_every)
+        a->snap.resize(2 * checkpoint_every);
+    a->lastKept = true;
+    size_t keptBytes = 0;
     for (int s = 0; s < nsteps; ++s)
     {
         if (s % checkpoint_every == 0)
@@ -1658,8 +1683,20 @@ int avbd_adjoint_forward(AvbdContext *ctx, int32_t nsteps, int32_t checkpoint_ev
             a->nKeys += ctx->nMan;
         }
         // step s is taped: its replay runs while the next FP32 step proceeds
+        SegSnap *keep = nullptr;
+        if (s >= lastStep && a->lastKept)
+        {
+            const TapeStep &ts = a->tape[s];
+            keptBytes += snap_bytes(n, ts.nMan, ts.iterations);
+            a->lastKept = keptBytes <= LAST_SEGMENT_BYTES;
+            if (a->lastKept)
+            {
+                keep = &a->snap[(lastSeg & 1) * checkpoint_every + (s - lastStep)];
+                CHECK(snap_reserve(ctx, *keep, n, ts.nMan, ts.iterations));
+            }
+        }
         CHECK(side_after_main(ctx));
-        CHECK(replay_step(ctx, s, nullptr));
+        CHECK(replay_step(ctx, s, keep));
     }
     CHECK(save_replay(ctx, a->last, a->tape.back().nMan));
     CHECK(main_after_side(ctx));
@@ -1852,7 +1889,12 @@ int avbd_adjoint_backward(AvbdContext *ctx, const double *d_position3, const dou
         CU(cudaEventRecord(a->evRep[set], a->side));
         return AVBD_OK;
     };
-    CHECK(replay_segment(nck - 1));
+    if (a->lastKept)
+        CU(cudaEventRecord(a->evRep[(nck - 1) & 1], a->side)); // the forward's snapshots are there
+    else
+        CHECK(replay_segment(nck - 1));
+    if (nck > 2)
+        a->lastKept = false; // its set is filled again below
     for (int seg = nck - 1; seg >= 0; --seg)
     {
         int set = seg & 1;
