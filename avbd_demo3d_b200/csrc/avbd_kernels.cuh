@@ -3994,16 +3994,20 @@ AVBD_DEV void st_relaxed_u64(unsigned long long *p, unsigned long long v)
 // warp finds for each of them the lane its chain starts from and the distance (pointer
 // doubling, five shuffles) and colours all of them in the pass after that lane, instead of a
 // link a pass. Measured: 64 uneven worlds with jointed chains up to 1,168 links 304 -> 65 us, 512
-// worlds (up to 2,026 links) 583 -> 126, 262,144 boxes in stacks 82 -> 77.
+// worlds (up to 2,026 links) 583 -> 118. Adjacency entries and rows are read four and eight
+// at a time, a load of all of them before the next load that depends on it: 262,144 boxes in
+// stacks 82 -> 54, 65,536 36 -> 26.
 //
 // The same cooperative launch then places the vertices in colour order, ascending body
 // index inside each colour (what sorting (colour, body) keys gives): block b counts the
 // colours of its contiguous share of the bodies, and after a grid barrier every block
 // derives its colours' write positions from all blocks' counts and writes the solve list,
 // the solve entries (body, row range) and each row's dual-owner / later-partner bits.
-constexpr int COLOUR_FLOW_BLOCK = 256;
+// Three blocks to an SM: 80 registers a thread without spills (two blocks leave chains more
+// batches per warp: 512 worlds 138 us against 118; four 128).
+constexpr int COLOUR_FLOW_BLOCK = 256, COLOUR_FLOW_RESIDENT = 3;
 
-__global__ void __launch_bounds__(COLOUR_FLOW_BLOCK) k_colour_greedy(
+__global__ void __launch_bounds__(COLOUR_FLOW_BLOCK, COLOUR_FLOW_RESIDENT) k_colour_greedy(
     DevBodies B, DevForces F, int n, unsigned long long *state, unsigned epoch, int *colour, ColourControl *ctl,
     StepCounters *cnt, unsigned spinLimit, int *blockCounts, int *colourStart, int *solveList, int4 *entries,
     const int *rowStart, StepState *st)
@@ -4025,6 +4029,7 @@ __global__ void __launch_bounds__(COLOUR_FLOW_BLOCK) k_colour_greedy(
     // another warp is polled (without blocking) in memory once per round. A warp that makes
     // no progress in a round backs off, and after spinLimit such rounds the wait has expired.
     constexpr int NB = 8; // lower-index neighbours kept in registers (more: rescanned per round)
+    constexpr int AHEAD = 4; // entries whose loads are in flight together
     for (int base = blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < n && !failed; base += stride)
     {
         const int v = base + lane;
@@ -4043,34 +4048,52 @@ __global__ void __launch_bounds__(COLOUR_FLOW_BLOCK) k_colour_greedy(
             if (!pending)
                 __stcg(&colour[v], -1);
             else
-                for (int k = F.adjStart[v]; k < F.adjStart[v + 1]; ++k)
+            {
+                const int end = F.adjStart[v + 1];
+                for (int k0 = F.adjStart[v]; k0 < end; k0 += AHEAD)
                 {
-                    unsigned e = F.adj[k];
-                    if (adj_type(e) == ADJ_IGNORE)
-                        continue;
-                    int2 ab = force_bodies(F, e);
-                    int u = ab.x == v ? ab.y : ab.x;
-                    // static bodies are not vertices; a dynamic neighbour shares this force
-                    if (u < 0 || u >= v || B.massMoment[u].x <= 0)
-                        continue;
-                    bool known = false; // another force of the same two bodies
+                    // AHEAD entries at a time, each load of all of them before the next one's
+                    unsigned e[AHEAD];
+                    int u[AHEAD];
 #pragma unroll
-                    for (int j = 0; j < NB; ++j)
-                        known = known || (j < nnb && nb[j] == u);
-                    if (known)
-                        continue;
-                    if (nnb < NB)
+                    for (int j = 0; j < AHEAD; ++j)
+                        e[j] = k0 + j < end ? F.adj[k0 + j] : make_adj(ADJ_IGNORE, 0u, 0u);
+#pragma unroll
+                    for (int j = 0; j < AHEAD; ++j)
                     {
-                        if (u >= base)
-                            intra |= 1u << nnb;
-#pragma unroll
-                        for (int j = 0; j < NB; ++j)
-                            nb[j] = j == nnb ? u : nb[j];
-                        ++nnb;
+                        int2 ab = make_int2(-1, -1);
+                        if (adj_type(e[j]) != ADJ_IGNORE)
+                            ab = force_bodies(F, e[j]);
+                        u[j] = ab.x == v ? ab.y : ab.x;
                     }
-                    else
-                        many = true;
+#pragma unroll
+                    for (int j = 0; j < AHEAD; ++j)
+                        // static bodies are not vertices; a dynamic neighbour shares this force
+                        if (u[j] >= v || (u[j] >= 0 && B.massMoment[u[j]].x <= 0))
+                            u[j] = -1;
+#pragma unroll
+                    for (int j = 0; j < AHEAD; ++j)
+                    {
+                        bool known = u[j] < 0; // or another force of the same two bodies
+#pragma unroll
+                        for (int i = 0; i < NB; ++i)
+                            known = known || (i < nnb && nb[i] == u[j]);
+                        if (known)
+                            continue;
+                        if (nnb < NB)
+                        {
+                            if (u[j] >= base)
+                                intra |= 1u << nnb;
+#pragma unroll
+                            for (int i = 0; i < NB; ++i)
+                                nb[i] = i == nnb ? u[j] : nb[i];
+                            ++nnb;
+                        }
+                        else
+                            many = true;
+                    }
                 }
+            }
         }
         const unsigned all = (1u << nnb) - 1u;
         // one lower neighbour, a lane of this warp: `from` the lane its chain starts from
@@ -4086,12 +4109,18 @@ __global__ void __launch_bounds__(COLOUR_FLOW_BLOCK) k_colour_greedy(
             intra = 0u;
         // shuffle passes look at the first kIntra neighbours (the warp's largest in-warp one)
         const int kIntra = __reduce_max_sync(0xFFFFFFFFu, 32 - __clz((int)intra));
+        auto use = [&](int c) { // constant indices: `used` stays in registers
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                used[j] |= (c >> 6) == j ? 1ull << (c & 63) : 0ull;
+        };
         // takes the smallest colour no lower neighbour uses; `state` is written at the end of
         // the round, by all lanes that took one together (one release for the warp)
         auto take = [&]() {
-            int c = 0;
-            while (c < 256 && ((used[c >> 6] >> (c & 63)) & 1ull))
-                c++;
+            int c = 256;
+#pragma unroll
+            for (int j = 3; j >= 0; --j)
+                c = used[j] != ~0ull ? 64 * j + __ffsll((long long)~used[j]) - 1 : c;
             if (c >= 256)
             {
                 cnt->error = DERR_TOO_MANY_COLOURS;
@@ -4111,18 +4140,18 @@ __global__ void __launch_bounds__(COLOUR_FLOW_BLOCK) k_colour_greedy(
             bool progressed = false;
             if (pending && !many)
             {
-                // neighbours in other warps
+                // neighbours in other warps: every word is asked for before the first is used
+                unsigned long long word[NB];
+#pragma unroll
+                for (int k = 0; k < NB; ++k)
+                    word[k] = link || k >= nnb || (((seen | intra) >> k) & 1u) ? 0ull : ld_relaxed_u64(&state[nb[k]]);
 #pragma unroll
                 for (int k = 0; k < NB; ++k)
                 {
-                    if (link || k >= nnb || (((seen | intra) >> k) & 1u))
+                    if ((word[k] >> 32) != (unsigned long long)epoch) // epochs are never 0
                         continue;
-                    const unsigned long long su = ld_relaxed_u64(&state[nb[k]]);
-                    if ((su >> 32) != (unsigned long long)epoch)
-                        continue;
-                    const int cu = (int)(su & 0xFFFFu), ru = (int)((su >> 16) & 0xFFFFu);
-                    if (cu < 256)
-                        used[cu >> 6] |= 1ull << (cu & 63);
+                    const int cu = (int)(word[k] & 0xFFFFu), ru = (int)((word[k] >> 16) & 0xFFFFu);
+                    use(cu);
                     round = max(round, ru + 1);
                     seen |= 1u << k;
                 }
@@ -4149,8 +4178,7 @@ __global__ void __launch_bounds__(COLOUR_FLOW_BLOCK) k_colour_greedy(
                         break;
                     }
                     const int cu = (int)(su & 0xFFFFu), ru = (int)((su >> 16) & 0xFFFFu);
-                    if (cu < 256)
-                        used[cu >> 6] |= 1ull << (cu & 63);
+                    use(cu);
                     round = max(round, ru + 1);
                 }
                 if (ready)
@@ -4174,7 +4202,7 @@ __global__ void __launch_bounds__(COLOUR_FLOW_BLOCK) k_colour_greedy(
                     if (pending && !many && in && !((seen >> k) & 1u) && cr != ~0u)
                     {
                         const int cu = (int)(cr & 0xFFFFu);
-                        used[cu >> 6] |= 1ull << (cu & 63);
+                        use(cu);
                         round = max(round, (int)(cr >> 16) + 1);
                         seen |= 1u << k;
                     }
@@ -4344,16 +4372,28 @@ __global__ void __launch_bounds__(COLOUR_FLOW_BLOCK) k_colour_greedy(
             const int r0 = rowStart[v], r1 = rowStart[v + 1];
             entries[pos] = make_int4(v, r0, r1, 0);
             // the rows whose contact or joint dual update this body owns in the fused pass
-            for (int r = r0; r < r1; ++r)
+            for (int ra = r0; ra < r1; ra += 2 * AHEAD)
             {
-                int2 row = F.rows[r];
-                const int p = row_partner(row);
-                const int cp = p >= 0 ? __ldcg(&colour[p]) : -1;
-                const bool own = p < 0 || cp < 0 || c < cp;
-                const bool later = p >= 0 && cp >= 0 && c < cp;
-                row.y = own ? (row.y | ROW_OWNS_DUAL) : (row.y & ~ROW_OWNS_DUAL);
-                row.y = later ? (row.y | ROW_PARTNER_LATER) : (row.y & ~ROW_PARTNER_LATER);
-                F.rows[r] = row;
+                int2 row[2 * AHEAD];
+                int cp[2 * AHEAD];
+#pragma unroll
+                for (int j = 0; j < 2 * AHEAD; ++j)
+                    row[j] = ra + j < r1 ? F.rows[ra + j] : make_int2(0, 0);
+#pragma unroll
+                for (int j = 0; j < 2 * AHEAD; ++j)
+                {
+                    const int p = row_partner(row[j]);
+                    cp[j] = p >= 0 ? __ldcg(&colour[p]) : -1;
+                }
+#pragma unroll
+                for (int j = 0; j < 2 * AHEAD; ++j)
+                {
+                    const bool own = cp[j] < 0 || c < cp[j], later = cp[j] >= 0 && c < cp[j];
+                    row[j].y &= ~(ROW_OWNS_DUAL | ROW_PARTNER_LATER);
+                    row[j].y |= (own ? ROW_OWNS_DUAL : 0) | (later ? ROW_PARTNER_LATER : 0);
+                    if (ra + j < r1)
+                        F.rows[ra + j] = row[j];
+                }
             }
         }
     }
