@@ -124,6 +124,7 @@ struct AvbdContext
     unsigned cellHashMask = 0, largeHashMask = 0;
     DArr<unsigned long long> bpKeys, bpKeysAlt;
     DArr<int> pairCount, pairOffset;
+    DArr<float4> entrySphere; // bounding spheres in the sorted grid entries' order
     DArr<int> pairRecorded; // BP_SLOTS new partners per grid entry lane from the counting pass
     DArr<int> pairLaneCount; // new partners per grid entry lane
     // LBVH broadphase mode: Morton-sorted binned bodies, tree nodes, grid position per body
@@ -1184,7 +1185,7 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
                 k_ll_chunk_bounds<<<grid_for(nL, 128), 128, 0, s>>>(G, ctx->large.p, ctx->largeSphere.p, nL,
                                                                     ctx->llChunkLo.p, ctx->llChunkHi.p);
                 LAUNCHED();
-                k_bp_large_large<BP_COUNT><<<grid_for(nItems, 128), 128, 0, s>>>(
+                k_bp_large_large<BP_COUNT><<<std::min(grid_for(nItems, 128), TALLY_BLOCKS), 128, 0, s>>>(
                     F, ctx->large.p, ctx->largeSphere.p, ctx->llItems.p, nItems, ctx->llCount.p, nullptr, 0, 0, cnt,
                     nullptr, ctx->llChunkLo.p, ctx->llChunkHi.p, ctx->llRecorded.p, S);
                 LAUNCHED();
@@ -1218,7 +1219,8 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
             CHECK(ensure_temp(ctx, bytes));
             CU(cub::DeviceRadixSort::SortKeys(ctx->cubTemp.p, bytes, dk, nB, 24, gridEnd, M));
             ctx->launches++;
-            k_bp_hash_runs<<<grid_for(nB, 256), 256, 0, M>>>(dk.Current(), nB, cell_hash(ctx));
+            CHECK(reserve(ctx, ctx->entrySphere, (size_t)nB, false));
+            k_bp_hash_runs<<<grid_for(nB, 256), 256, 0, M>>>(dk.Current(), nB, cell_hash(ctx), B, ctx->entrySphere.p);
             LAUNCHED();
             CHECK(reserve(ctx, ctx->pairRecorded, (size_t)nB * BP_LANES * BP_SLOTS, false));
             CHECK(reserve(ctx, ctx->pairLaneCount, (size_t)nB * BP_LANES, false));
@@ -1226,10 +1228,10 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
                 CU(cudaStreamWaitEvent(M, evLists, 0));
             CU(cudaStreamWaitEvent(M, evPairSet, 0));
             // LBVH mode: the grid pass counts the large-body part only; the tree finds the rest
-            k_bp_pairs<BP_COUNT><<<grid_for((long long)nB * BP_LANES, 128), 128, 0, M>>>(
-                B, F, G, dk.Current(), nB, cell_hash(ctx), ctx->large.p, ctx->largeLo.p, ctx->largeHi.p,
-                ctx->largeSorted, large_hash(ctx), dt, ctx->pairCount.p, nullptr, 0, 0, cnt, ctx->pairRecorded.p,
-                ctx->pairLaneCount.p, nullptr, S, lbvh ? (1u << 14) : 0x7FFFu);
+            k_bp_pairs<BP_COUNT><<<std::min(grid_for((long long)nB * BP_LANES, 128), TALLY_BLOCKS), 128, 0, M>>>(
+                B, F, G, dk.Current(), ctx->entrySphere.p, nB, cell_hash(ctx), ctx->large.p, ctx->largeLo.p,
+                ctx->largeHi.p, nL ? ctx->largeSorted : nullptr, nL * LARGE_MAX_CELLS, large_hash(ctx), dt,
+                ctx->pairCount.p, nullptr, 0, 0, cnt, ctx->pairRecorded.p, ctx->pairLaneCount.p, nullptr, S, lbvh ? (1u << 14) : 0x7FFFu);
             LAUNCHED();
             if (lbvh)
             {
@@ -1302,9 +1304,9 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
             if (entryBlocks + llBlocks > 0)
             {
                 k_bp_emit<<<entryBlocks + llBlocks, 128, 0, ctx->stream>>>(
-                    B, F, G, dk.Current(), nB, cell_hash(ctx), ctx->large.p, ctx->largeLo.p, ctx->largeHi.p,
-                    ctx->largeSorted, large_hash(ctx), dt, ctx->pairCount.p, ctx->pairOffset.p, cnt,
-                    ctx->pairRecorded.p, ctx->pairLaneCount.p, st, S, entryBlocks, ctx->largeSphere.p, ctx->llItems.p,
+                    B, F, G, dk.Current(), ctx->entrySphere.p, nB, cell_hash(ctx), ctx->large.p, ctx->largeLo.p,
+                    ctx->largeHi.p, nL ? ctx->largeSorted : nullptr, nL * LARGE_MAX_CELLS, large_hash(ctx), dt,
+                    ctx->pairCount.p, ctx->pairOffset.p, cnt, ctx->pairRecorded.p, ctx->pairLaneCount.p, st, S, entryBlocks, ctx->largeSphere.p, ctx->llItems.p,
                     nItems, ctx->llCount.p, ctx->llOffset.p, ctx->llChunkLo.p, ctx->llChunkHi.p, ctx->llRecorded.p);
                 LAUNCHED();
             }
@@ -1346,8 +1348,9 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
         {
             // the pairs each entry recorded while counting; entries that found more search again
             k_bp_pairs<BP_EMIT_RECORDED><<<grid_for((long long)nB * BP_LANES, 128), 128, 0, ctx->stream>>>(
-                B, F, G, dk.Current(), nB, cell_hash(ctx), ctx->large.p, ctx->largeLo.p, ctx->largeHi.p,
-                ctx->largeSorted, large_hash(ctx), dt, ctx->pairCount.p, ctx->pairOffset.p, M0,
+                B, F, G, dk.Current(), ctx->entrySphere.p, nB, cell_hash(ctx), ctx->large.p, ctx->largeLo.p,
+                ctx->largeHi.p, nL ? ctx->largeSorted : nullptr, nL * LARGE_MAX_CELLS, large_hash(ctx), dt,
+                ctx->pairCount.p, ctx->pairOffset.p, M0,
                 (unsigned long long)ctx->nextSeq, cnt, ctx->pairRecorded.p, ctx->pairLaneCount.p, nullptr, S);
             LAUNCHED();
         }
@@ -2644,7 +2647,7 @@ void avbd_destroy(AvbdContext *ctx)
     adjoint_release(ctx);
     for (DArr<float4> *a : {&ctx->pos, &ctx->quat, &ctx->initLin, &ctx->initAng, &ctx->inertLin, &ctx->inertAng,
                             &ctx->dqLin, &ctx->dqAng, &ctx->initAngInv, &ctx->inertAngInv,
-                            &ctx->bodyFlow, &ctx->contactFlow, &ctx->jointFlow, &ctx->massDt2,
+                            &ctx->bodyFlow, &ctx->contactFlow, &ctx->jointFlow, &ctx->massDt2, &ctx->entrySphere,
                             &ctx->vel, &ctx->angvel, &ctx->prevVel, &ctx->massMoment, &ctx->sizeRad, &ctx->largeLo,
                             &ctx->largeHi, &ctx->largeSphere, &ctx->spring, &ctx->joint[0], &ctx->joint[1]})
         release(*a);
