@@ -73,7 +73,7 @@ def test_wide_iterations_match_oracle(gpu, name):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("nx,ny,height", [(31, 66, 16), (32, 64, 16)])  # 32,737 and 32,769 bodies
+@pytest.mark.parametrize("nx,ny,height", [(19, 503, 3), (28, 64, 16)])  # 28,672 and 28,673 bodies
 def test_both_sides_of_the_body_limit(gpu, nx, ny, height):
     scene = scenes.stack_grid(nx, ny, height, seed=3)
     a, b = World(scene), World(scene)
