@@ -1208,7 +1208,20 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
         };
         // keys -> sorted entries -> cell runs -> counted new pairs, on the context stream;
         // the pair set and (waitLists) the large bodies' cell lists are waited for first
-        auto counting_pass = [&](bool waitLists) -> int {
+        // one block grids a small world (a device step's, in the grid mode)
+        const bool small = deviceCounts && !lbvh && ctx->W == 1 && nB > 0 && nB <= 4 * SMALL_GRID_BLOCK &&
+                           nL <= SMALL_GRID_LARGE;
+        const int largeTotal = small ? nL : nL * LARGE_MAX_CELLS; // entries of the sorted large keys
+        auto small_grid = [&]() -> int {
+            CHECK(reserve(ctx, ctx->entrySphere, (size_t)nB, false));
+            auto kernel = nB <= SMALL_GRID_BLOCK ? k_grid_small<1> : k_grid_small<4>;
+            kernel<<<1, SMALL_GRID_BLOCK, 0, M>>>(B, G, ctx->binned.p, nB, dt, ctx->bpKeys.p, ctx->entrySphere.p,
+                                                 cell_hash(ctx), nL, ctx->largeKeys.p, large_hash(ctx));
+            LAUNCHED();
+            dk = cub::DoubleBuffer<unsigned long long>(ctx->bpKeys.p, ctx->bpKeysAlt.p);
+            return AVBD_OK;
+        };
+        auto sort_entries = [&]() -> int {
             k_bp_keys<<<grid_for(nB, 256), 256, 0, M>>>(B, G, ctx->binned.p, nB, ctx->bpKeys.p);
             LAUNCHED();
             dk = cub::DoubleBuffer<unsigned long long>(ctx->bpKeys.p, ctx->bpKeysAlt.p);
@@ -1225,15 +1238,19 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
             CHECK(reserve(ctx, ctx->entrySphere, (size_t)nB, false));
             k_bp_hash_runs<<<grid_for(nB, 256), 256, 0, M>>>(dk.Current(), nB, cell_hash(ctx), B, ctx->entrySphere.p);
             LAUNCHED();
+            return AVBD_OK;
+        };
+        auto counting_pass = [&](bool waitLists) -> int {
+            CHECK(small ? small_grid() : sort_entries());
             CHECK(reserve(ctx, ctx->pairRecorded, (size_t)nB * BP_LANES * BP_SLOTS, false));
             CHECK(reserve(ctx, ctx->pairLaneCount, (size_t)nB * BP_LANES, false));
             if (waitLists)
                 CU(cudaStreamWaitEvent(M, evLists, 0));
-            CU(cudaStreamWaitEvent(M, evPairSet, 0));
+            CU(cudaStreamWaitEvent(M, evPairSet, 0)); // the pair set and the large bodies' boxes
             // LBVH mode: the grid pass counts the large-body part only; the tree finds the rest
             k_bp_pairs<BP_COUNT><<<std::min(grid_for((long long)nB * BP_LANES, 128), TALLY_BLOCKS), 128, 0, M>>>(
                 B, F, G, dk.Current(), ctx->entrySphere.p, nB, cell_hash(ctx), ctx->large.p, ctx->largeLo.p,
-                ctx->largeHi.p, nL ? ctx->largeSorted : nullptr, nL * LARGE_MAX_CELLS, large_hash(ctx), dt,
+                ctx->largeHi.p, nL ? ctx->largeSorted : nullptr, largeTotal, large_hash(ctx), dt,
                 ctx->pairCount.p, nullptr, 0, 0, cnt, ctx->pairRecorded.p, ctx->pairLaneCount.p, nullptr, S, lbvh ? (1u << 14) : 0x7FFFu);
             LAUNCHED();
             if (lbvh)
@@ -1267,18 +1284,21 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
         ctx->largeSorted = ctx->largeKeys.p;
         if (nB)
         {
-            k_bp_bounds<<<std::min(grid_for(nB, 256), 148 * 2), 256, 0, M>>>(B, G, ctx->binned.p, nB, dt);
-            LAUNCHED();
-            k_bp_params<<<grid_for(ctx->W, 128), 128, 0, M>>>(G, ctx->worldBinned.p);
-            LAUNCHED();
-            if (nL || lbvh)
-                CU(cudaEventRecord(evParams, M));
-            if (nL)
+            if (!small)
             {
-                CU(cudaStreamWaitEvent(S2, evParams, 0));
-                CU(cudaStreamWaitEvent(S2, evLarge, 0));
-                CHECK(large_cell_lists(ctx, nL, S2, ctx->cubTempSide[1]));
-                CU(cudaEventRecord(evLists, S2));
+                k_bp_bounds<<<std::min(grid_for(nB, 256), 148 * 2), 256, 0, M>>>(B, G, ctx->binned.p, nB, dt);
+                LAUNCHED();
+                k_bp_params<<<grid_for(ctx->W, 128), 128, 0, M>>>(G, ctx->worldBinned.p);
+                LAUNCHED();
+                if (nL || lbvh)
+                    CU(cudaEventRecord(evParams, M));
+                if (nL)
+                {
+                    CU(cudaStreamWaitEvent(S2, evParams, 0));
+                    CU(cudaStreamWaitEvent(S2, evLarge, 0));
+                    CHECK(large_cell_lists(ctx, nL, S2, ctx->cubTempSide[1]));
+                    CU(cudaEventRecord(evLists, S2));
+                }
             }
             if (lbvh) // the tree needs only the grid parameters and the bodies
             {
@@ -1286,7 +1306,7 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
                 CHECK(lbvh_build(ctx, nB, S3));
                 CU(cudaEventRecord(evTree, S3));
             }
-            CHECK(counting_pass(nL > 0));
+            CHECK(counting_pass(nL > 0 && !small));
         }
         CU(cudaStreamWaitEvent(M, evLL, 0)); // join: everything side[0] made
         if (deviceCounts)
@@ -1308,7 +1328,7 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
             {
                 k_bp_emit<<<entryBlocks + llBlocks, 128, 0, ctx->stream>>>(
                     B, F, G, dk.Current(), ctx->entrySphere.p, nB, cell_hash(ctx), ctx->large.p, ctx->largeLo.p,
-                    ctx->largeHi.p, nL ? ctx->largeSorted : nullptr, nL * LARGE_MAX_CELLS, large_hash(ctx), dt,
+                    ctx->largeHi.p, nL ? ctx->largeSorted : nullptr, largeTotal, large_hash(ctx), dt,
                     ctx->pairCount.p, ctx->pairOffset.p, cnt, ctx->pairRecorded.p, ctx->pairLaneCount.p, st, S, entryBlocks, ctx->largeSphere.p, ctx->llItems.p,
                     nItems, ctx->llCount.p, ctx->llOffset.p, ctx->llChunkLo.p, ctx->llChunkHi.p, ctx->llRecorded.p);
                 LAUNCHED();
@@ -1352,7 +1372,7 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
             // the pairs each entry recorded while counting; entries that found more search again
             k_bp_pairs<BP_EMIT_RECORDED><<<grid_for((long long)nB * BP_LANES, 128), 128, 0, ctx->stream>>>(
                 B, F, G, dk.Current(), ctx->entrySphere.p, nB, cell_hash(ctx), ctx->large.p, ctx->largeLo.p,
-                ctx->largeHi.p, nL ? ctx->largeSorted : nullptr, nL * LARGE_MAX_CELLS, large_hash(ctx), dt,
+                ctx->largeHi.p, nL ? ctx->largeSorted : nullptr, largeTotal, large_hash(ctx), dt,
                 ctx->pairCount.p, ctx->pairOffset.p, M0,
                 (unsigned long long)ctx->nextSeq, cnt, ctx->pairRecorded.p, ctx->pairLaneCount.p, nullptr, S);
             LAUNCHED();
