@@ -1206,11 +1206,9 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
             }
             return AVBD_OK;
         };
-        // keys -> sorted entries -> cell runs -> counted new pairs, on the context stream;
-        // the pair set and (waitLists) the large bodies' cell lists are waited for first
-        // one block grids a small world (a device step's, in the grid mode)
-        const bool small = deviceCounts && !lbvh && ctx->W == 1 && nB > 0 && nB <= 4 * SMALL_GRID_BLOCK &&
-                           nL <= SMALL_GRID_LARGE;
+        // one block grids a small world (a device step's, in the grid mode): k_grid_small says
+        // why up to 4,096 entries
+        const bool small = deviceCounts && !lbvh && ctx->W == 1 && nB > 0 && nB <= 4 * SMALL_GRID_BLOCK;
         const int largeTotal = small ? nL : nL * LARGE_MAX_CELLS; // entries of the sorted large keys
         auto small_grid = [&]() -> int {
             CHECK(reserve(ctx, ctx->entrySphere, (size_t)nB, false));
@@ -1240,6 +1238,8 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
             LAUNCHED();
             return AVBD_OK;
         };
+        // keys -> sorted entries -> cell runs -> counted new pairs, on the context stream;
+        // the pair set and (waitLists) the large bodies' cell lists are waited for first
         auto counting_pass = [&](bool waitLists) -> int {
             CHECK(small ? small_grid() : sort_entries());
             CHECK(reserve(ctx, ctx->pairRecorded, (size_t)nB * BP_LANES * BP_SLOTS, false));

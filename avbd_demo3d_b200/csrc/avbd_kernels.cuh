@@ -661,15 +661,16 @@ __global__ void k_bp_hash_large_runs(const unsigned long long *keys, int n, Hash
 }
 
 // The grid of one world of up to 1,024 ITEMS binned bodies in one block: bounds, parameters, keys,
-// their sort, runs and spheres, which otherwise are five launches around a library sort, 22 to
-// 48 us of the step's chain. Measured, rollouts of one to four steps: 210-box pyramid 275 ->
-// 255 us, 1,000 boxes 546 -> 452, 3,000 mixed bodies 650 -> 571, 4,096 boxes 1139 -> 999. At
-// eight entries a thread the block is slower than the launches (6,000 mixed bodies 710 ->
-// 804), so 4,096 entries are the most it takes. The sort orders (cell, place in the binned list) pairs by
+// their sort, runs and spheres, which otherwise are five launches around a library sort, 22 us
+// (210-box pyramid) to 46 us (4,096 boxes) of kernels in the step's chain. It is bound by the
+// latency of that chain. Per rollout of one to four steps, launches -> one block, medians on one
+// GPU: pyramid 275 -> 255 us, 1,000 boxes 546 -> 452, 3,000 mixed bodies 650 -> 571, 4,096 boxes
+// 1139 -> 999. Eight entries a thread (6,000 mixed bodies) lost about 9% against the launches, so
+// 4,096 entries are the most it takes. The sort orders (cell, place in the binned list) pairs by
 // the cell bits the grid uses; it is stable, so a cell's entries stay in body order. The world's
-// large bodies (at most SMALL_GRID_LARGE) all go on its global list, in order: an entry's
-// sixteen lanes test a few hundred faster than cell lists are built and sorted.
-constexpr int SMALL_GRID_BLOCK = 1024, SMALL_GRID_LARGE = 512;
+// large bodies (a twentieth at most, so 215 here) all go on its global list, in order: an
+// entry's sixteen lanes test so few without cell lists to build and sort.
+constexpr int SMALL_GRID_BLOCK = 1024;
 
 template <int ITEMS>
 __global__ void __launch_bounds__(SMALL_GRID_BLOCK) k_grid_small(DevBodies B, DevGrid G, const int *binned, int nBinned,

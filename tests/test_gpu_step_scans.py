@@ -12,9 +12,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("nx,ny,height,steps", [
     (1, 1, 1, 4), (1, 2, 1, 4), (2, 1, 5, 4),
-    (7, 9, 17, 4), (7, 9, 18, 4),      # 1,024 grid entries, about: below and above (one block
-    (17, 17, 15, 3), (16, 18, 15, 3),  # grids up to 4,096, one or four entries a thread)
-    (16, 16, 16, 4),
+    (16, 16, 16, 4),    # one tile of grid entries, about
     (16, 20, 16, 3),    # 32,768 force-list entries (with the spare manifolds), about: below
     (18, 18, 16, 3),    # and above
     (25, 26, 16, 3),    # 32,768 manifolds with the spare ones, about: below
