@@ -353,6 +353,13 @@ void release(DArr<T> &a)
 
 int grid_for(long long n, int block) { return (int)std::max<long long>(1, (n + block - 1) / block); }
 
+// Blocks of 128 threads of a pass that counts pairs (TALLY_BLOCKS says why not one per 128).
+int tally_grid(long long threads)
+{
+    const int blocks = grid_for(threads, 128);
+    return std::min(blocks, std::max(TALLY_BLOCKS, blocks / TALLY_ROUNDS));
+}
+
 int ensure_temp(AvbdContext *ctx, size_t bytes) { return reserve(ctx, ctx->cubTemp, bytes, false); }
 
 // Phase timing with CUDA events on the context stream (enabled by avbd_set_profiling).
@@ -1188,7 +1195,7 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
                 k_ll_chunk_bounds<<<grid_for(nL, 128), 128, 0, s>>>(G, ctx->large.p, ctx->largeSphere.p, nL,
                                                                     ctx->llChunkLo.p, ctx->llChunkHi.p);
                 LAUNCHED();
-                k_bp_large_large<BP_COUNT><<<std::min(grid_for(nItems, 128), TALLY_BLOCKS), 128, 0, s>>>(
+                k_bp_large_large<BP_COUNT><<<tally_grid(nItems), 128, 0, s>>>(
                     F, ctx->large.p, ctx->largeSphere.p, ctx->llItems.p, nItems, ctx->llCount.p, nullptr, 0, 0, cnt,
                     nullptr, ctx->llChunkLo.p, ctx->llChunkHi.p, ctx->llRecorded.p, S);
                 LAUNCHED();
@@ -1248,7 +1255,7 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
                 CU(cudaStreamWaitEvent(M, evLists, 0));
             CU(cudaStreamWaitEvent(M, evPairSet, 0)); // the pair set and the large bodies' boxes
             // LBVH mode: the grid pass counts the large-body part only; the tree finds the rest
-            k_bp_pairs<BP_COUNT><<<std::min(grid_for((long long)nB * BP_LANES, 128), TALLY_BLOCKS), 128, 0, M>>>(
+            k_bp_pairs<BP_COUNT><<<tally_grid((long long)nB * BP_LANES), 128, 0, M>>>(
                 B, F, G, dk.Current(), ctx->entrySphere.p, nB, cell_hash(ctx), ctx->large.p, ctx->largeLo.p,
                 ctx->largeHi.p, nL ? ctx->largeSorted : nullptr, largeTotal, large_hash(ctx), dt,
                 ctx->pairCount.p, nullptr, 0, 0, cnt, ctx->pairRecorded.p, ctx->pairLaneCount.p, nullptr, S, lbvh ? (1u << 14) : 0x7FFFu);

@@ -784,12 +784,15 @@ AVBD_DEV void warp_add(unsigned long long *dst, unsigned v)
 // What a counting pass adds up: checks, sphere hits, hits already linked. One address takes
 // about one atomic a nanosecond, so the passes go round their work with a few blocks per SM
 // and add once per block and counter instead of once per warp (broadphase of 262,144 boxes,
-// 400,000 additions a step before: 667 -> 610 us; 65,536 boxes 232 -> 217).
+// 400,000 additions a step before: 667 -> 610 us; 65,536 boxes 232 -> 217). Beyond TALLY_ROUNDS
+// rounds a block the shares become too unequal where the worlds of a batch are (the broadphase
+// alone of 4,096 worlds, 1.4 million bodies: 2.53 ms in 77 rounds, 2.28 in 12), so larger
+// passes launch more blocks.
 struct PairTally
 {
     unsigned checks = 0, hits = 0, cons = 0;
 };
-constexpr int TALLY_BLOCKS = 148 * 16; // the most blocks of 128 threads a counting pass launches
+constexpr int TALLY_BLOCKS = 148 * 16, TALLY_ROUNDS = 12; // blocks of 128 threads of a counting pass
 
 AVBD_DEV void block_tally(StepCounters *cnt, const PairTally &t)
 {
@@ -1008,20 +1011,24 @@ AVBD_DEV void bp_pairs(long long tid, const DevBodies &B, const DevForces &F, co
                 recorded[slot0 + found] = bIdx;
             found++;
         };
-        // the entries from j on that belong to a run, four keys and spheres in flight
+        // The entries from j on that belong to a run, four keys and spheres in flight. An emission
+        // searches only where a lane found more than it could record: one at a time there, or the
+        // four set the registers of all its lanes (52, and 32 so: the broadphase alone of 4,096
+        // worlds, which emits every pair, 2.63 -> 2.53 ms).
+        constexpr int AHEAD = EMIT ? 1 : 4;
         auto search = [&](int j, unsigned long long run) {
-            for (;; j += 4)
+            for (;; j += AHEAD)
             {
-                unsigned long long kj[4];
-                float4 sj[4];
+                unsigned long long kj[AHEAD];
+                float4 sj[AHEAD];
 #pragma unroll
-                for (int u = 0; u < 4; ++u)
+                for (int u = 0; u < AHEAD; ++u)
                 {
                     kj[u] = j + u < nBinned ? keys[j + u] : HASH_EMPTY;
                     sj[u] = spheres[min(j + u, nBinned - 1)];
                 }
 #pragma unroll
-                for (int u = 0; u < 4; ++u)
+                for (int u = 0; u < AHEAD; ++u)
                 {
                     if (j + u >= nBinned || (kj[u] >> 24) != run)
                         return;
@@ -1115,14 +1122,13 @@ AVBD_DEV void bp_pairs(long long tid, const DevBodies &B, const DevForces &F, co
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(128) k_bp_pairs(DevBodies B, DevForces F, DevGrid G, const unsigned long long *keys,
-                                                  const float4 *spheres, int nBinned, HashTable cells, const int *large,
-                                                  const float4 *largeLo, const float4 *largeHi,
-                                                  const unsigned long long *largeKeys, int largeTotal,
-                                                  HashTable largeCells, float dt, int *counts, const int *offsets, int base, unsigned long long seqBase,
-                                                  StepCounters *cnt, int *recorded, int *laneCounts,
-                                                  const StepState *st = nullptr, PairSet S = PairSet(),
-                                                  unsigned partMask = 0x7FFFu)
+__global__ void __launch_bounds__(128, MODE == BP_COUNT ? 0 : 16)
+    k_bp_pairs(DevBodies B, DevForces F, DevGrid G, const unsigned long long *keys, const float4 *spheres, int nBinned,
+               HashTable cells, const int *large, const float4 *largeLo, const float4 *largeHi,
+               const unsigned long long *largeKeys, int largeTotal, HashTable largeCells, float dt, int *counts,
+               const int *offsets, int base, unsigned long long seqBase, StepCounters *cnt, int *recorded,
+               int *laneCounts, const StepState *st = nullptr, PairSet S = PairSet(),
+               unsigned partMask = 0x7FFFu)
 {
     PairTally tally;
     const long long stride = (long long)gridDim.x * blockDim.x;
@@ -1590,7 +1596,7 @@ __global__ void k_bp_large_large(DevForces F, const int *large, const float4 *la
 
 // A device step's emission: the grid entries' new pairs, and after their blocks the large
 // bodies'.
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, 16)
     k_bp_emit(DevBodies B, DevForces F, DevGrid G, const unsigned long long *keys, const float4 *spheres, int nBinned,
               HashTable cells,
               const int *large, const float4 *largeLo, const float4 *largeHi, const unsigned long long *largeKeys,
