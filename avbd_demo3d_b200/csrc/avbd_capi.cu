@@ -1095,12 +1095,9 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
         CHECK(reserve(ctx, ctx->bpKeysAlt, n, false));
         CHECK(reserve(ctx, ctx->sapVals, n, false));
         CHECK(reserve(ctx, ctx->sapValsAlt, n, false));
-        if (n > INT_MAX / SAP_PARTS)
-            return fail(ctx, AVBD_ERR_CAPACITY, "too many bodies (%d) for the sweep-and-prune broadphase", n);
-        const int items = SAP_PARTS * n;
-        const int sweepBlocks = grid_for(32ll * items, SAP_BLOCK);
-        CHECK(reserve(ctx, ctx->pairCount, items, false));
-        CHECK(reserve(ctx, ctx->pairOffset, items, false));
+        const int sweepBlocks = grid_for(n, SAP_WARPS);
+        CHECK(reserve(ctx, ctx->pairCount, n, false));
+        CHECK(reserve(ctx, ctx->pairOffset, n, false));
         k_sap_axis<<<W, SAP_TILE, 0, ctx->stream>>>(B, ctx->worldStart.p, ctx->sapAxis.p);
         LAUNCHED();
         k_sap_keys<<<grid_for(n, 256), 256, 0, ctx->stream>>>(B, ctx->bodyWorld.p, ctx->sapAxis.p, ctx->bpKeys.p,
@@ -1117,23 +1114,23 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
         CU(cub::DeviceRadixSort::SortPairs(ctx->cubTemp.p, bytes, dk, dv, n, 0, endBit, ctx->stream));
         ctx->launches++;
         DevForces F = dev_forces(ctx);
-        k_sap_sweep<false><<<sweepBlocks, SAP_BLOCK, 0, ctx->stream>>>(B, F, ctx->sapAxis.p, dk.Current(), dv.Current(),
-                                                                       n, ctx->pairCount.p, nullptr, 0, 0, cnt);
+        k_sap_sweep<false><<<sweepBlocks, SAP_BLOCK, 0, ctx->stream>>>(
+            B, F, ctx->sapAxis.p, ctx->worldStart.p, dk.Current(), dv.Current(), n, ctx->pairCount.p, nullptr, 0, 0, cnt);
         LAUNCHED();
-        CHECK(scan_counts(ctx, ctx->pairCount.p, ctx->pairOffset.p, items, 0));
+        CHECK(scan_counts(ctx, ctx->pairCount.p, ctx->pairOffset.p, n, 0));
         ctx->launches++;
         if (deviceCounts)
         {
-            k_bp_commit<<<1, 1, 0, ctx->stream>>>(ctx->stepState.p, ctx->pairOffset.p, ctx->pairCount.p, items, nullptr,
+            k_bp_commit<<<1, 1, 0, ctx->stream>>>(ctx->stepState.p, ctx->pairOffset.p, ctx->pairCount.p, n, nullptr,
                                                   nullptr, 0, nullptr, cnt, (long long)man_capacity(ctx));
             LAUNCHED();
             k_sap_sweep<true><<<sweepBlocks, SAP_BLOCK, 0, ctx->stream>>>(
-                B, dev_forces(ctx), ctx->sapAxis.p, dk.Current(), dv.Current(), n, nullptr, ctx->pairOffset.p, 0, 0, cnt,
-                ctx->stepState.p);
+                B, dev_forces(ctx), ctx->sapAxis.p, ctx->worldStart.p, dk.Current(), dv.Current(), n, ctx->pairCount.p,
+                ctx->pairOffset.p, 0, 0, cnt, ctx->stepState.p);
             LAUNCHED();
             return AVBD_OK;
         }
-        k_total<<<1, 1, 0, ctx->stream>>>(ctx->pairOffset.p, ctx->pairCount.p, items, ctx->hScalars);
+        k_total<<<1, 1, 0, ctx->stream>>>(ctx->pairOffset.p, ctx->pairCount.p, n, ctx->hScalars);
         LAUNCHED();
         CU(cudaStreamSynchronize(ctx->stream));
         CHECK(nonfinite_checked(ctx));
@@ -1143,8 +1140,8 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
             CHECK(reserve_manifolds(ctx, ctx->man[ctx->cur], (size_t)(M0 + P1), (size_t)M0));
             DevForces F2 = dev_forces(ctx);
             k_sap_sweep<true><<<sweepBlocks, SAP_BLOCK, 0, ctx->stream>>>(
-                B, F2, ctx->sapAxis.p, dk.Current(), dv.Current(), n, nullptr, ctx->pairOffset.p, M0,
-                (unsigned long long)ctx->nextSeq, cnt);
+                B, F2, ctx->sapAxis.p, ctx->worldStart.p, dk.Current(), dv.Current(), n, ctx->pairCount.p,
+                ctx->pairOffset.p, M0, (unsigned long long)ctx->nextSeq, cnt);
             LAUNCHED();
         }
     }

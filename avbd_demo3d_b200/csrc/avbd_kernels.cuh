@@ -1748,18 +1748,56 @@ __global__ void k_sap_keys(DevBodies B, const int *bodyWorld, const int *axis, u
 // past its maximum; bounding-sphere hits become new manifolds (A = interval i's body,
 // B = the later one) unless the bodies are already constrained, in sweep order.
 //
-// An interval's candidates are one stretch of the sorted keys (minima ascend, so the first that
-// starts past the maximum ends it, found by a 32-way search), cut into SAP_PARTS parts of a
-// warp each: the ground's interval holds every body of its world, and one thread walking it was
-// most of a step (1,860 bodies: 2.9 ms a step, 0.29 now that no thread walks and the step
-// keeps its counts on the device). counts[SAP_PARTS i + part] keep the sweep's order through the scan.
-constexpr int SAP_PARTS = 32, SAP_BLOCK = 256;
+// An interval's candidates are one stretch of its world's sorted keys: minima ascend, so the
+// first that starts past the maximum ends it (looked for among the next 32, then by a 32-way
+// search). A warp takes an interval of up to SAP_ALONE candidates; a longer one is left to its
+// block's 32 warps together, since the ground's interval holds every body of its world and one
+// warp walking it would be the step. counts[i] keep the sweep's order through the scan.
+// Bound by the latency of a warp's loads in one world, by issue in large batches. A step by a
+// thread an interval / by 32 warps an interval / so (us): 4,096 worlds of 7 bodies 730 / 1,085 /
+// 665, of 37 bodies 2,390 / 4,710 / 2,330; 64 uneven worlds 4,950 / 1,553 / 1,015; one world of
+// 1,860 bodies 3,040 / 267 / 254, of 20,737 30,460 / 997 / 787. SAP_ALONE at 128 / 512 / 2,048:
+// 1,860 bodies 282 / 255 / 361, 512 worlds 1,943 / 1,882 / 2,041, 65,537 bodies 2,088 / 2,050 /
+// 1,864 a step.
+constexpr int SAP_BLOCK = 1024, SAP_WARPS = SAP_BLOCK / 32, SAP_ALONE = 512, SAP_AHEAD = 4;
+static_assert(SAP_WARPS == 32, "a warp's lanes stand for the block's warps");
+
+AVBD_DEV int sap_end(const unsigned long long *keys, int first, int last, unsigned long long top, int lane)
+{
+    constexpr unsigned ALL = 0xFFFFFFFFu;
+    const int next = __popc(__ballot_sync(ALL, first + lane < last && keys[first + lane] <= top));
+    if (next < 32)
+        return first + next;
+    int lo = first + 32, hi = last; // keys[lo - 1] <= top < keys[hi]
+    while (lo < hi)
+    {
+        const int step = (hi - lo + 31) / 32, at = lo + lane * step;
+        const int below = __popc(__ballot_sync(ALL, at < hi && keys[at] <= top));
+        // probes 0 .. below - 1 are inside: the end lies in (last inside, first outside]
+        hi = min(hi, lo + below * step);
+        lo = below > 0 ? lo + (below - 1) * step + 1 : hi;
+    }
+    return hi;
+}
+
+// Candidate b of body a: a new pair?
+AVBD_DEV bool sap_test(const DevForces &F, int a, float3 pa, float ra, int b, float3 pb, float rb, PairTally &tally)
+{
+    const float3 dp = sub(pa, pb);
+    const float r = ra + rb;
+    if (dot(dp, dp) > r * r)
+        return false;
+    const bool con = constrained(F, a, b);
+    tally.hits++;
+    tally.cons += con;
+    return !con;
+}
 
 template <bool EMIT>
 __global__ void __launch_bounds__(SAP_BLOCK) k_sap_sweep(DevBodies B, DevForces F, const int *axis,
-                                                         const unsigned long long *keys, const int *vals, int n,
-                                                         int *counts, const int *offsets, int base,
-                                                         unsigned long long seqBase, StepCounters *cnt,
+                                                         const int *worldStart, const unsigned long long *keys,
+                                                         const int *vals, int n, int *counts, const int *offsets,
+                                                         int base, unsigned long long seqBase, StepCounters *cnt,
                                                          const StepState *st = nullptr)
 {
     constexpr unsigned ALL = 0xFFFFFFFFu;
@@ -1770,89 +1808,116 @@ __global__ void __launch_bounds__(SAP_BLOCK) k_sap_sweep(DevBodies B, DevForces 
         base = st->manBase;
         seqBase = st->seqBase;
     }
-    __shared__ int hitSum, consSum;
-    if (!EMIT)
+    __shared__ int longEnd[SAP_WARPS], longFound[SAP_WARPS], tileFound[2][SAP_WARPS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int i0 = (int)blockIdx.x * SAP_WARPS, i = i0 + warp;
+    const unsigned lower = (1u << lane) - 1u;
+    PairTally tally;
+    auto emit = [&](int m, int a, int b) {
+        F.man.ab[m] = make_int2(a, b);
+        F.man.seq[m] = seqBase + (unsigned long long)(m - base);
+        F.man.n[m] = 0;
+    };
+    int forBlock = 0;
+    if (i < n && (!EMIT || counts[i] > 0)) // warp-uniform
     {
-        if (threadIdx.x == 0)
-            hitSum = consSum = 0;
-        __syncthreads();
-    }
-    const int lane = threadIdx.x & 31;
-    const long long item = ((long long)blockIdx.x * SAP_BLOCK + threadIdx.x) >> 5;
-    const int i = (int)(item / SAP_PARTS), part = (int)(item % SAP_PARTS);
-    if (i < n) // warp-uniform
-    {
-        const unsigned world = (unsigned)(keys[i] >> 32);
-        const int a = vals[i];
+        const int world = (int)(keys[i] >> 32), a = vals[i];
         const float3 pa = xyz(B.pos[a]);
         const float ra = B.sizeRad[a].w;
-        // the first key past (world, maximum); a maximum of -0 counts as +0, as in a comparison
+        // the last key inside is at most (world, maximum); a maximum of -0 counts as +0, as in a comparison
         const float ahi = comp(pa, axis[world]) + ra + 0.0f;
         const unsigned long long top = ((unsigned long long)world << 32) | float_order(ahi);
-        int lo = i + 1, hi = n; // keys[lo - 1] <= top < keys[hi]
-        while (lo < hi)
+        const int end = sap_end(keys, i + 1, worldStart[world + 1], top, lane);
+        if (!EMIT && lane == 0)
+            tally.checks += (unsigned)(end - (i + 1));
+        if (end - (i + 1) > SAP_ALONE)
+            forBlock = end;
+        else
         {
-            const int step = (hi - lo + 31) / 32, at = lo + lane * step;
-            const int below = __popc(__ballot_sync(ALL, at < hi && keys[at] <= top));
-            // probes 0 .. below - 1 are inside: the end lies in (last inside, first outside]
-            hi = min(hi, lo + below * step);
-            lo = below > 0 ? lo + (below - 1) * step + 1 : hi;
+            int found = 0;
+            const int out = EMIT ? base + offsets[i] : 0;
+            for (int at = i + 1; at < end; at += 32 * SAP_AHEAD)
+            {
+                const int rounds = (end - at + 31) / 32; // of the SAP_AHEAD, those that hold a candidate
+                int b[SAP_AHEAD];
+                float4 pb[SAP_AHEAD];
+                float rb[SAP_AHEAD];
+#pragma unroll
+                for (int u = 0; u < SAP_AHEAD; ++u)
+                    if (u < rounds)
+                        b[u] = vals[min(at + 32 * u + lane, end - 1)];
+#pragma unroll
+                for (int u = 0; u < SAP_AHEAD; ++u)
+                    if (u < rounds)
+                    {
+                        pb[u] = B.pos[b[u]];
+                        rb[u] = B.sizeRad[b[u]].w;
+                    }
+#pragma unroll
+                for (int u = 0; u < SAP_AHEAD; ++u)
+                {
+                    if (u >= rounds)
+                        break;
+                    const bool fresh =
+                        at + 32 * u + lane < end && sap_test(F, a, pa, ra, b[u], xyz(pb[u]), rb[u], tally);
+                    const unsigned mask = __ballot_sync(ALL, fresh);
+                    if (EMIT && fresh)
+                        emit(out + found + __popc(mask & lower), a, b[u]);
+                    found += __popc(mask);
+                }
+            }
+            if (!EMIT && lane == 0)
+                counts[i] = found;
         }
-        const int len = hi - (i + 1), chunk = (len + SAP_PARTS * 32 - 1) / (SAP_PARTS * 32) * 32;
-        const int j0 = i + 1 + part * chunk, j1 = min(j0 + chunk, hi);
-        int found = 0, hits = 0, cons = 0;
-        const int out = EMIT && j0 < j1 ? base + offsets[item] : 0;
-        for (int at = j0; at < j1; at += 32)
+    }
+    if (lane == 0)
+    {
+        longEnd[warp] = forBlock;
+        longFound[warp] = 0;
+    }
+    __syncthreads();
+    int tile = 0;
+    for (unsigned longs = __ballot_sync(ALL, longEnd[lane] != 0); longs; longs &= longs - 1)
+    {
+        const int w = __ffs((int)longs) - 1, end = longEnd[w];
+        const int a = vals[i0 + w];
+        const float3 pa = xyz(B.pos[a]);
+        const float ra = B.sizeRad[a].w;
+        int out = EMIT ? base + offsets[i0 + w] : 0;
+        for (int at = i0 + w + 1; at < end; at += SAP_BLOCK)
         {
-            const int j = at + lane;
+            const int j = at + (int)threadIdx.x;
             bool fresh = false;
             int b = 0;
-            if (j < j1)
+            if (j < end)
             {
                 b = vals[j];
-                const float3 dp = sub(pa, xyz(B.pos[b]));
-                const float r = ra + B.sizeRad[b].w;
-                const bool hit = !(dot(dp, dp) > r * r);
-                const bool con = hit && constrained(F, a, b);
-                fresh = hit && !con;
-                hits += hit;
-                cons += con;
+                fresh = sap_test(F, a, pa, ra, b, xyz(B.pos[b]), B.sizeRad[b].w, tally);
             }
             const unsigned mask = __ballot_sync(ALL, fresh);
-            if (EMIT && fresh)
+            if (!EMIT)
             {
-                const int m = out + found + __popc(mask & ((1u << lane) - 1u));
-                F.man.ab[m] = make_int2(a, b);
-                F.man.seq[m] = seqBase + (unsigned long long)(m - base);
-                F.man.n[m] = 0;
+                if (lane == 0 && mask)
+                    atomicAdd(&longFound[w], __popc(mask));
+                continue;
             }
-            found += __popc(mask);
-        }
-        if (!EMIT)
-        {
+            int *found = tileFound[tile++ & 1]; // the other half is written before this one again
             if (lane == 0)
-            {
-                counts[item] = found;
-                if (part == 0 && len > 0)
-                    atomicAdd(&cnt->pairChecks, (unsigned long long)len);
-            }
-            hits = __reduce_add_sync(ALL, hits);
-            cons = __reduce_add_sync(ALL, cons);
-            if (lane == 0 && hits)
-            {
-                atomicAdd(&hitSum, hits);
-                atomicAdd(&consSum, cons);
-            }
+                found[warp] = __popc(mask);
+            __syncthreads();
+            const int all = found[lane];
+            const int before = __reduce_add_sync(ALL, lane < warp ? all : 0);
+            if (fresh)
+                emit(out + before + __popc(mask & lower), a, b);
+            out += __reduce_add_sync(ALL, all);
         }
     }
     if (!EMIT)
     {
         __syncthreads();
-        if (threadIdx.x == 0 && hitSum)
-        {
-            atomicAdd(&cnt->sphereHits, (unsigned long long)hitSum);
-            atomicAdd(&cnt->constrainedHits, (unsigned long long)consSum);
-        }
+        if (lane == 0 && forBlock != 0)
+            counts[i] = longFound[warp];
+        block_tally(cnt, tally);
     }
 }
 
