@@ -180,6 +180,7 @@ struct AvbdContext
     bool hasSpheres = false; // rolling friction pass after the velocity update
     int iterBlocks = 0;       // co-resident blocks of the iteration kernel (0: not launchable)
     int wideBlocks = 0;       // the same for the wide iteration kernel
+    bool wide = false;        // the running step iterates in the wide kernel (choose_wide)
     DArr<IterSync> iterSync;
     DArr<int> iterDone; // per body: iterations completed in the running iteration launch
     int *hIterError = nullptr; // pinned: barrier expiry of the last iteration kernel
@@ -428,7 +429,23 @@ int reserve_manifolds(AvbdContext *ctx, ManBuf &b, size_t count, size_t used)
 // 217, 20,480 155 and 222, 24,576 201 and 226, 31,744 250 and 235, 65,536 488 and 297; 64
 // uneven worlds (19,728 bodies) 134 and 310.
 constexpr int WIDE_MAX_BODIES = 28672;
-bool wide_iterations(const AvbdContext *ctx) { return ctx->wideBlocks > 0 && ctx->n <= WIDE_MAX_BODIES; }
+bool wide_possible(const AvbdContext *ctx) { return ctx->wideBlocks > 0 && ctx->n <= WIDE_MAX_BODIES; }
+
+// The choice for the step that begins. With a single colour nothing is handed over, and the
+// wide kernel is the better one only while its warps take one chunk each, four bodies (boxes in
+// one layer, wide and k_iterations: 6,400 53 and 61 us, 8,100 82 and 63, 16,900 127 and 73,
+// 27,889 180 and 94; the same with five pairs of boxes, two colours: 184 and 165, 12,100 91 and
+// 152). The colours are those of the last step the host has seen: settled, or, with steps
+// pending, what the newest finished one left in page-locked memory. Either kernel gives the
+// same bits, so an old count costs time alone.
+bool choose_wide(const AvbdContext *ctx)
+{
+    if (!wide_possible(ctx))
+        return false;
+    const int colours = ctx->pendingFast > 0 ? *(volatile const int *)&ctx->hState->nColours : ctx->nColours;
+    const int solved = ((volatile const int *)ctx->hColourStarts)[1];
+    return colours != 1 || solved <= ctx->wideBlocks * WIDE_WARPS * (32 / WIDE_MIN_GROUP);
+}
 
 DevBodies dev_bodies(AvbdContext *ctx)
 {
@@ -450,7 +467,7 @@ DevBodies dev_bodies(AvbdContext *ctx)
     B.massMoment = ctx->massMoment.p;
     B.massDt2 = ctx->massDt2.p;
     B.sizeRad = ctx->sizeRad.p;
-    B.flow = wide_iterations(ctx) ? ctx->bodyFlow.p : nullptr;
+    B.flow = ctx->wide ? ctx->bodyFlow.p : nullptr;
     B.shape = ctx->hasShapes ? ctx->shape.p : nullptr;
     B.friction = ctx->friction.p;
     return B;
@@ -487,7 +504,7 @@ DevForces dev_forces(AvbdContext *ctx)
     F.adj = ctx->adj.p;
     F.rowStart = ctx->rowStart.p;
     F.rows = ctx->rows.p;
-    const bool wide = wide_iterations(ctx);
+    const bool wide = ctx->wide;
     F.contactFlow = wide ? ctx->contactFlow.p : nullptr;
     F.jointFlow = wide ? ctx->jointFlow.p : nullptr;
     return F;
@@ -1434,7 +1451,7 @@ int init_old_manifolds(AvbdContext *ctx)
 // The wide iteration kernel's stamped words for `manifolds` manifolds and every joint.
 int flow_reserve(AvbdContext *ctx, size_t manifolds)
 {
-    if (!wide_iterations(ctx))
+    if (!ctx->wide)
         return AVBD_OK;
     CHECK(reserve(ctx, ctx->contactFlow, 16 * std::max<size_t>(manifolds, 1), false));
     return reserve(ctx, ctx->jointFlow, 4 * (size_t)std::max(ctx->nJoint, 1), false);
@@ -1646,7 +1663,7 @@ int init_forces(AvbdContext *ctx)
             LAUNCHED();
             ctx->jcur = o;
             ctx->nJoint = (int)newJ;
-            if (newJ && wide_iterations(ctx))
+            if (newJ && ctx->wide)
             {
                 k_joint_flow<<<grid_for(newJ, 128), 128, 0, ctx->stream>>>(dev_forces(ctx));
                 LAUNCHED();
@@ -1788,7 +1805,7 @@ int iterate_persistent(AvbdContext *ctx, bool deviceCounts = false, IterTape tap
     unsigned spinLimit = ctx->waitIteration ? ctx->waitIteration : ITER_SPIN_LIMIT;
     const StepState *st = deviceCounts ? ctx->stepState.p : nullptr;
     const int *orphans = &ctx->counters.p->orphans;
-    if (wide_iterations(ctx))
+    if (ctx->wide)
     {
         int *error = &sync->error;
         void *args[] = {&B,     &F,         &P,  &entries, &colourStart, &nColours, &iterations,
@@ -1877,6 +1894,7 @@ int iterate(AvbdContext *ctx)
 
 int step_once(AvbdContext *ctx)
 {
+    ctx->wide = choose_wide(ctx); // before any view of the buffers is taken
     // refuse non-finite body state before anything changes, like a device-resident step
     CU(cudaMemsetAsync(ctx->stepFlags.p, 0, sizeof(int), ctx->stream));
     CHECK(step_clear(ctx, ctx->stepFlags.p, false));
@@ -2000,6 +2018,7 @@ int device_reserve(AvbdContext *ctx)
 // capacity, with k_step_begin / k_bp_commit deciding on the device whether the step can run.
 int step_device(AvbdContext *ctx)
 {
+    ctx->wide = choose_wide(ctx); // before any view of the buffers is taken
     // with no step pending the host's counts are current (a settle, a synchronous step, a
     // load or an edit came last): they become the device state's
     if (ctx->stateDirty || (ctx->pendingFast == 0 && (ctx->nMan != ctx->stateMan || ctx->nextSeq != ctx->stateSeq ||
@@ -2385,7 +2404,7 @@ int upload_bodies(AvbdContext *ctx, const AvbdBodies *b, bool props)
             CHECK(reserve(ctx, *a, std::max(n, 1), false));
             CU(cudaMemsetAsync(a->p, 0, sizeof(float4) * std::max(n, 1), ctx->stream));
         }
-        if (wide_iterations(ctx))
+        if (wide_possible(ctx))
             CHECK(reserve(ctx, ctx->bodyFlow, (size_t)FLOW_STRIDE * std::max(n, 1), false));
         CU(cudaStreamSynchronize(ctx->stream));
     }
@@ -3057,7 +3076,7 @@ int avbd_load_batch(AvbdContext *ctx, int32_t num_worlds, const int32_t *world_s
     }
     CHECK(build_adjacency(ctx));
     CU(cudaStreamSynchronize(ctx->stream));
-    ctx->nColours = 0;
+    ctx->nColours = ctx->hState->nColours = 0;
     ctx->nSolve = 0;
     ctx->loaded = true;
     ctx->stateDirty = true;
