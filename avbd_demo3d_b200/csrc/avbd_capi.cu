@@ -11,6 +11,7 @@
 // progress, colour ranges) to size launches and buffers.
 #include "../../include/avbd_cuda.h"
 #include "avbd_kernels.cuh"
+#include "avbd_launch_shape.h"
 
 #include <cub/cub.cuh>
 
@@ -21,8 +22,6 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
-#include <map>
-#include <mutex>
 #include <string>
 #include <vector>
 
@@ -2530,21 +2529,17 @@ bool allow_iteration_smem()
     return ok;
 }
 
-// Co-resident blocks of the cooperative kernels, the same for every context of a device: asked
-// for once per device (the occupancy queries are a good part of a small world's creation).
-struct LaunchShape
+// The shape of a device's cooperative launches; false if a query failed.
+bool query_launch_shape(int device_ordinal, bool iterations, LaunchShape &shape)
 {
-    int colourBlocks = 1, colourFlowBlocks = 1, iterBlocks = 0, wideBlocks = 0;
-};
-
-LaunchShape query_launch_shape(int device_ordinal, bool iterations)
-{
-    LaunchShape shape;
     int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_ordinal);
-    auto per_sm = [](const void *kernel, int block, size_t smem) {
+    bool ok = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_ordinal) == cudaSuccess;
+    auto per_sm = [&ok](const void *kernel, int block, size_t smem) {
         int blocks = 0;
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, block, smem) == cudaSuccess ? blocks : 0;
+        const bool known =
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, block, smem) == cudaSuccess;
+        ok = ok && known;
+        return known ? blocks : 0;
     };
     shape.colourBlocks = std::max(1, sms * std::max(1, per_sm((const void *)k_colour_all, 256, 0)));
     // the greedy colouring: co-resident, and at most four blocks per SM (every block
@@ -2567,19 +2562,15 @@ LaunchShape query_launch_shape(int device_ordinal, bool iterations)
         shape.wideBlocks = wide > 0 ? sms : 0;
     }
     cudaGetLastError();
-    return shape;
+    return ok;
 }
 
 LaunchShape launch_shape(int device)
 {
-    const bool iterations = allow_iteration_smem();
-    static std::mutex lock;
-    static std::map<int, LaunchShape> known;
-    std::lock_guard<std::mutex> hold(lock);
-    auto it = known.find(device);
-    if (it == known.end())
-        it = known.emplace(device, query_launch_shape(device, iterations)).first;
-    return it->second;
+    static LaunchShapes shapes;
+    return shapes.of(device, allow_iteration_smem(), [device](bool iterations, LaunchShape &shape) {
+        return query_launch_shape(device, iterations, shape);
+    });
 }
 
 } // namespace
