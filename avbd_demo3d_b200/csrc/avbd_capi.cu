@@ -182,7 +182,7 @@ struct AvbdContext
     bool wide = false;        // the running step iterates in the wide kernel (choose_wide)
     DArr<IterSync> iterSync;
     DArr<int> iterDone; // per body: iterations completed in the running iteration launch
-    int *hIterError = nullptr; // pinned: barrier expiry of the last iteration kernel
+    int *hIterError = nullptr; // pinned: a wait of the last iteration kernel expired
     int colourMode = 0;       // 0 greedy (list-index priority), 1 hashed priority
     int *hColourSummary = nullptr; // pinned: vertices, rounds, max colour, error
     int *hColourStarts = nullptr;  // pinned: 257 colour range starts
@@ -1131,7 +1131,8 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
         ctx->launches++;
         DevForces F = dev_forces(ctx);
         k_sap_sweep<false><<<sweepBlocks, SAP_BLOCK, 0, ctx->stream>>>(
-            B, F, ctx->sapAxis.p, ctx->worldStart.p, dk.Current(), dv.Current(), n, ctx->pairCount.p, nullptr, 0, 0, cnt);
+            B, F, ctx->sapAxis.p, ctx->worldStart.p, dk.Current(), dv.Current(), n, ctx->pairCount.p, nullptr, 0, 0,
+            cnt);
         LAUNCHED();
         CHECK(scan_counts(ctx, ctx->pairCount.p, ctx->pairOffset.p, n, 0));
         ctx->launches++;
@@ -1271,7 +1272,8 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
             k_bp_pairs<BP_COUNT><<<tally_grid((long long)nB * BP_LANES), 128, 0, M>>>(
                 B, F, G, dk.Current(), ctx->entrySphere.p, nB, cell_hash(ctx), ctx->large.p, ctx->largeLo.p,
                 ctx->largeHi.p, nL ? ctx->largeSorted : nullptr, largeTotal, large_hash(ctx), dt,
-                ctx->pairCount.p, nullptr, 0, 0, cnt, ctx->pairRecorded.p, ctx->pairLaneCount.p, nullptr, S, lbvh ? (1u << 14) : 0x7FFFu);
+                ctx->pairCount.p, nullptr, 0, 0, cnt, ctx->pairRecorded.p, ctx->pairLaneCount.p, nullptr, S,
+                lbvh ? (1u << 14) : 0x7FFFu);
             LAUNCHED();
             if (lbvh)
             {
@@ -1349,8 +1351,8 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
                 k_bp_emit<<<entryBlocks + llBlocks, 128, 0, ctx->stream>>>(
                     B, F, G, dk.Current(), ctx->entrySphere.p, nB, cell_hash(ctx), ctx->large.p, ctx->largeLo.p,
                     ctx->largeHi.p, nL ? ctx->largeSorted : nullptr, largeTotal, large_hash(ctx), dt,
-                    ctx->pairCount.p, ctx->pairOffset.p, cnt, ctx->pairRecorded.p, ctx->pairLaneCount.p, st, S, entryBlocks, ctx->largeSphere.p, ctx->llItems.p,
-                    nItems, ctx->llCount.p, ctx->llOffset.p, ctx->llChunkLo.p, ctx->llChunkHi.p, ctx->llRecorded.p);
+                    ctx->pairCount.p, ctx->pairOffset.p, cnt, ctx->pairRecorded.p, ctx->pairLaneCount.p, st, S,
+                    entryBlocks, ctx->largeSphere.p, ctx->llItems.p, nItems, ctx->llCount.p, ctx->llOffset.p, ctx->llChunkLo.p, ctx->llChunkHi.p, ctx->llRecorded.p);
                 LAUNCHED();
             }
             return AVBD_OK;
@@ -1765,7 +1767,7 @@ int colour_readback(AvbdContext *ctx)
     CU(cudaMemcpyAsync(ctx->hCounters, ctx->counters.p, sizeof(StepCounters), cudaMemcpyDeviceToHost, ctx->stream));
     CU(cudaStreamSynchronize(ctx->stream));
     if (*ctx->hIterError)
-        return fail(ctx, AVBD_ERR_STATE, "iteration kernel wait expired (a grid barrier or a partner body's iteration count)");
+        return fail(ctx, AVBD_ERR_STATE, "iteration kernel wait expired (a partner body's iteration)");
     const int *sum = ctx->hColourSummary; // vertices, rounds, maxColour, error
     if (sum[3])
         return fail(ctx, AVBD_ERR_STATE, "colouring did not finish (barrier wait expired or round cap reached)");
@@ -2130,7 +2132,7 @@ int settle(AvbdContext *ctx)
     {
         if (s.error == STEP_ERR_ITERATION)
             return fail(ctx, AVBD_ERR_STATE,
-                        "iteration kernel wait expired (a grid barrier or a partner body's iteration count)");
+                        "iteration kernel wait expired (a partner body's iteration)");
         if (s.error == STEP_ERR_COLOURS)
             return fail(ctx, AVBD_ERR_CAPACITY, "constraint graph needs more than 256 colours");
         return fail(ctx, AVBD_ERR_STATE, "colouring did not finish (barrier wait expired or round cap reached)");
@@ -3286,7 +3288,7 @@ int avbd_synchronize(AvbdContext *ctx)
     SETTLED();
     CU(cudaStreamSynchronize(ctx->stream));
     if (*ctx->hIterError)
-        return fail(ctx, AVBD_ERR_STATE, "iteration kernel wait expired (a grid barrier or a partner body's iteration count)");
+        return fail(ctx, AVBD_ERR_STATE, "iteration kernel wait expired (a partner body's iteration)");
     return AVBD_OK;
 }
 

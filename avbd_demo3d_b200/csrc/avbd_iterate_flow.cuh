@@ -1,5 +1,5 @@
 // All iterations of a step in one launch for worlds whose colours leave the chip mostly idle:
-// each body is solved by 8 to 32 lanes of one warp, and warps hand bodies to one another
+// each body is solved by 8 or 32 lanes of one warp, and warps hand bodies to one another
 // through stamped 16-byte words.
 //
 // What bounds such a world is the chain from one colour's bodies to the next colour's, not
@@ -17,7 +17,7 @@
 //    column side by side.
 // Every float operation and the order of every sum are those of primal_batch and
 // ldl_solve27, so the results are the same bits. Measured against k_iterations (us for the 10
-// iterations of a step): a 20-link rope 172 -> 67, the 210-box pyramid 404 -> 75, 6,000 mixed
+// iterations of a step): a 20-link rope 172 -> 67, the 210-box pyramid 404 -> 85, 6,000 mixed
 // bodies 303 -> 115, 4,096 boxes in stacks 202 -> 65, 20,000 poured spheres (3,950 solved) 385
 // -> 120, 64 uneven worlds (13,700 solved) 292 -> 129.
 //
@@ -47,7 +47,8 @@
 namespace avbd
 {
 
-// One block per SM of 16 warps: 128 registers a thread, which the words in flight need.
+// One block per SM of 12 warps: up to 168 registers a thread (the instances take 162 to 165, none
+// spills), which the words in flight need.
 constexpr int WIDE_BLOCK = 384, WIDE_WARPS = WIDE_BLOCK / 32, WIDE_MIN_GROUP = 8;
 
 struct WideShared

@@ -54,7 +54,7 @@ struct DevBodies
     float4 *initAngInv, *inertAngInv;
     float4 *massMoment, *sizeRad;
     float4 *massDt2; // massMoment / dt^2, the diagonal of every solve's M/dt^2 (k_warm_start)
-    // the narrow-world iteration kernel's stamped body words (avbd_iterate_flow.cuh); null
+    // the wide iteration kernel's stamped body words (avbd_iterate_flow.cuh); null
     // where that kernel does not run
     float4 *flow;
     float *friction;
@@ -90,7 +90,7 @@ struct DevForces
     // the constraint rows each body's primal solve stamps, in force order (rows_listed)
     int *rowStart; // n + 1
     int2 *rows;    // (force-list entry, (partner body + 1) << 3 | row of that force)
-    // stamped multiplier words of the narrow-world iteration kernel: 16 float4 per manifold,
+    // stamped multiplier words of the wide iteration kernel: 16 float4 per manifold,
     // 4 per joint (avbd_iterate_flow.cuh)
     float4 *contactFlow, *jointFlow;
 };
@@ -150,7 +150,7 @@ enum StepError
     STEP_ERR_NONE = 0,
     STEP_ERR_COLOURING = 1,     // the colouring's barrier wait expired or it ran out of rounds
     STEP_ERR_COLOURS = 2,       // the constraint graph needs more than 256 colours
-    STEP_ERR_ITERATION = 3      // a grid barrier or partner wait of the iteration kernel expired
+    STEP_ERR_ITERATION = 3      // a partner wait of the iteration kernel expired
 };
 
 struct StepState
@@ -831,8 +831,8 @@ constexpr int LARGE_HITS = 48; // large bodies within an entry's reach that its 
 
 template <int MODE>
 AVBD_DEV void bp_pairs(long long tid, const DevBodies &B, const DevForces &F, const DevGrid &G,
-                       const unsigned long long *keys, const float4 *spheres, int nBinned, HashTable cells, const int *large,
-                       const float4 *largeLo, const float4 *largeHi, const unsigned long long *largeKeys,
+                       const unsigned long long *keys, const float4 *spheres, int nBinned, HashTable cells,
+                       const int *large, const float4 *largeLo, const float4 *largeHi, const unsigned long long *largeKeys,
                        int largeTotal, HashTable largeCells, float dt, int *counts, const int *offsets, int base,
                        unsigned long long seqBase, StepCounters *cnt, int *recorded, int *laneCounts,
                        const StepState *st, PairSet S, unsigned partMask, PairTally &tally)
@@ -893,9 +893,10 @@ AVBD_DEV void bp_pairs(long long tid, const DevBodies &B, const DevForces &F, co
     {
         // The large bodies (lane 14's part) by the entry's sixteen lanes: fast or many large
         // bodies fill a cell's list and the world's global one (20,000 poured spheres: up to a
-        // thousand an entry; the step's broadphase 527 us on one lane, 176 so). Each list is tested sixteen at a time; the
-        // hits, few, are put in large-index order (the merged order of the two lists) and
-        // then looked up and recorded side by side. More hits than LARGE_HITS: lane 14 alone.
+        // thousand an entry; the step's broadphase 527 us on one lane, 176 so). Each list is
+        // tested sixteen at a time; the hits, few, are put in large-index order (the merged
+        // order of the two lists) and then looked up and recorded side by side. More hits than
+        // LARGE_HITS: lane 14 alone.
         __shared__ int hitIndex[128 / BP_LANES][LARGE_HITS], hitSorted[128 / BP_LANES][LARGE_HITS];
         const unsigned group = 0xFFFFu << ((threadIdx.x & 31) & ~(BP_LANES - 1));
         const unsigned below = group & ((1u << (threadIdx.x & 31)) - 1u);
@@ -930,7 +931,8 @@ AVBD_DEV void bp_pairs(long long tid, const DevBodies &B, const DevForces &F, co
                     {
                         l = (int)(v & 0xFFFFFFull);
                         const float4 lo = largeLo[l], hi = largeHi[l];
-                        const float3 q = f3(rclamp(ac.x, lo.x, hi.x), rclamp(ac.y, lo.y, hi.y), rclamp(ac.z, lo.z, hi.z));
+                        const float3 q =
+                            f3(rclamp(ac.x, lo.x, hi.x), rclamp(ac.y, lo.y, hi.y), rclamp(ac.z, lo.z, hi.z));
                         const float3 dp = sub(ac, q);
                         const float reach = sa.w + aslack + lo.w + margin4;
                         isHit = !(dot(dp, dp) > reach * reach);
@@ -1598,18 +1600,17 @@ __global__ void k_bp_large_large(DevForces F, const int *large, const float4 *la
 // bodies'.
 __global__ void __launch_bounds__(128, 16)
     k_bp_emit(DevBodies B, DevForces F, DevGrid G, const unsigned long long *keys, const float4 *spheres, int nBinned,
-              HashTable cells,
-              const int *large, const float4 *largeLo, const float4 *largeHi, const unsigned long long *largeKeys,
-              int largeTotal, HashTable largeCells, float dt, int *counts, const int *offsets, StepCounters *cnt, int *recorded,
-              int *laneCounts, const StepState *st, PairSet S, int entryBlocks, const float4 *largeSphere,
+              HashTable cells, const int *large, const float4 *largeLo, const float4 *largeHi,
+              const unsigned long long *largeKeys, int largeTotal, HashTable largeCells, float dt, int *counts,
+              const int *offsets, StepCounters *cnt, int *recorded, int *laneCounts, const StepState *st, PairSet S, int entryBlocks, const float4 *largeSphere,
               const int4 *items, int nItems, int *llCounts, const int *llOffsets, const uint4 *chunkLo,
               const uint4 *chunkHi, int *llRecorded)
 {
     PairTally tally; // counted before
     if ((int)blockIdx.x < entryBlocks)
-        bp_pairs<BP_EMIT_RECORDED>((long long)blockIdx.x * blockDim.x + threadIdx.x, B, F, G, keys, spheres, nBinned, cells,
-                                   large, largeLo, largeHi, largeKeys, largeTotal, largeCells, dt, counts, offsets, 0, 0, cnt,
-                                   recorded, laneCounts, st, S, 0x7FFFu, tally);
+        bp_pairs<BP_EMIT_RECORDED>((long long)blockIdx.x * blockDim.x + threadIdx.x, B, F, G, keys, spheres, nBinned,
+                                   cells, large, largeLo, largeHi, largeKeys, largeTotal, largeCells, dt, counts,
+                                   offsets, 0, 0, cnt, recorded, laneCounts, st, S, 0x7FFFu, tally);
     else
         bp_large_large<BP_EMIT_RECORDED>((blockIdx.x - entryBlocks) * blockDim.x + threadIdx.x, F, large, largeSphere,
                                          items, nItems, llCounts, llOffsets, 0, 0, cnt, st, chunkLo, chunkHi,
@@ -2299,10 +2300,10 @@ struct ContactRec
     bool stick;
 };
 
-// Loads of state that other blocks of one persistent launch write between its grid
-// barriers (poses, pose differences, contact and joint multipliers and penalties) go to L2
-// (ld.global.cg) there, so no block reads a stale L1 line after a barrier. Kernels that
-// end before the state changes again use plain loads.
+// Loads of state that other blocks of one persistent launch write while it runs (poses, pose
+// differences, contact and joint multipliers and penalties) go to L2 (ld.global.cg) there, so
+// no block reads a stale L1 line after its wait. Kernels that end before the state changes
+// again use plain loads.
 template <bool COH>
 AVBD_DEV float4 ld_state(const float4 *p)
 {
@@ -3020,7 +3021,7 @@ __global__ void k_step_begin(DevBodies B, const float4 *joint, int nJoint, StepS
 // Body warm start (solver.cpp:1134-1169)
 // ---------------------------------------------------------------------------
 
-// Stamped words of a body in the narrow-world iteration kernel (avbd_iterate_flow.cuh): its
+// Stamped words of a body in the wide iteration kernel (avbd_iterate_flow.cuh): its
 // orientation, pose difference and position, three floats and a stamp in each 16-byte word.
 // Six words a body (the last unused) keep the words a contact reads in two 32-byte sectors.
 constexpr int FLOW_STRIDE = 6, FLOW_USED = 5;
@@ -3804,9 +3805,9 @@ AVBD_DEV void unit_sync()
         asm volatile("bar.sync %0, %1;" ::"r"(1 + (int)threadIdx.x / SUB), "n"(SUB) : "memory");
 }
 
-// Per-body progress of the iteration kernel when it runs without per-colour grid barriers:
-// done[b] = the iterations body b has completed in this launch. `done` null: the
-// barriers order the passes and nothing is waited for.
+// Per-body progress of the iteration kernel: done[b] = the iterations body b has completed in
+// this launch. `done` null: the per-colour form, whose launches order the passes, so nothing
+// is waited for.
 struct IterFlow
 {
     int *done = nullptr;
@@ -4234,7 +4235,7 @@ __global__ void __launch_bounds__(BLOCK, 1) k_iterations(DevBodies B, DevForces 
 {
     if (st)
     {
-        if (step_aborted(st)) // uniform: every block leaves before the first barrier
+        if (step_aborted(st)) // uniform: every block leaves at once
             return;
         nColours = st->nColours;
         F.nMan = st->nMan;
@@ -4443,7 +4444,7 @@ __global__ void __launch_bounds__(COLOUR_FLOW_BLOCK, COLOUR_FLOW_RESIDENT) k_col
                 used[j] |= (c >> 6) == j ? 1ull << (c & 63) : 0ull;
         };
         // takes the smallest colour no lower neighbour uses; `state` is written at the end of
-        // the round, by all lanes that took one together (one release for the warp)
+        // the round, by all lanes that took one together (one relaxed store instruction)
         auto take = [&]() {
             int c = 256;
 #pragma unroll

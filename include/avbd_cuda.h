@@ -254,18 +254,18 @@ int avbd_write_bodies(AvbdContext *ctx, const AvbdBodies *bodies);
 
 /* Solver::step() for nsteps steps (solver.cpp:934-937 via stepCpuReference 1036-1041).
  * Asynchronous on the context stream. In AVBD_STEP_DEVICE mode (the default, for the grid,
- * LBVH and sweep-and-prune broadphases with the single-launch iterations) a step keeps every count it needs on the
- * device and returns as soon as its launches are issued. A step that cannot run as issued
- * stops on the device before it changes anything, and so does every step issued after
- * it: new pairs that do not fit the manifold buffers, a grid that needs the reference's
+ * LBVH and sweep-and-prune broadphases with the single-launch iterations) a step keeps every
+ * count it needs on the device and returns as soon as its launches are issued. A step that
+ * cannot run as issued stops on the device before it changes anything, and so does every step
+ * issued after it: new pairs that do not fit the manifold buffers, a grid that needs the reference's
  * cell-count cap (rescaled with the host's cbrtf), a joint broken in an earlier step (its
  * removal is compacted on the host). The next call that waits for the device (a read,
  * avbd_synchronize, avbd_get_stats, an edit) redoes those steps synchronously, so results
  * are always the same bits. In AVBD_STEP_HOST mode every step reads its counts on the host.
  * Errors of a step surface at the next call that waits for the device and latch:
- * AVBD_ERR_STATE when a bounded wait expires (a grid barrier, a row waiting for its
- * partner body's iteration count, the colouring's barrier) and when a body's position,
- * orientation or velocity is not finite at the start of a step (the step refuses it and
+ * AVBD_ERR_STATE when a bounded wait expires (a row waiting for its partner body's
+ * iteration, the colouring's barrier and words) and when a body's position, orientation or
+ * velocity is not finite at the start of a step (the step refuses it and
  * leaves the world as it was). */
 int avbd_step(AvbdContext *ctx, int32_t nsteps);
 /* Wait for the context stream (and redo or report any device-resident step, as above). */
@@ -316,9 +316,9 @@ int avbd_set_step_mode(AvbdContext *ctx, int32_t mode);
  * bounding spheres overlap without touching get a manifold that lasts one step); a small spare
  * makes steps that create many pairs stop on the device and be redone on the host. */
 int avbd_set_manifold_headroom(AvbdContext *ctx, int64_t spare);
-/* Poll limits of the bounded waits: the colouring's grid barrier and the iteration
- * kernel's grid barriers and partner waits (0 = the defaults, 2^24 and 2^22 polls). A wait
- * that reaches its limit makes the step fail with AVBD_ERR_STATE, as described at
+/* Poll limits of the bounded waits: the colouring's (its grid barrier and the words passed
+ * between its warps) and the iteration kernels' waits for partner bodies (0 = the defaults,
+ * 2^24 and 2^22 polls). A wait that reaches its limit makes the step fail with AVBD_ERR_STATE, as described at
  * avbd_step; the context stays usable after avbd_clear_error and a reload. No counterpart
  * in the reference (its CPU solver never waits). */
 int avbd_set_wait_limits(AvbdContext *ctx, uint32_t colouring_polls, uint32_t iteration_polls);
@@ -371,12 +371,12 @@ int avbd_snapshot_json(AvbdContext *ctx, uint64_t frame, const char *scene_name,
                        int64_t capacity, int64_t *size);
 
 /* Iteration mode: AVBD_ITERATIONS_PERSISTENT (default) runs every iteration of a step in
- * one cooperative launch with grid-wide barriers between colours and each contact's dual
- * update fused into the next iteration's primal row of the body that owns it;
+ * one cooperative launch, in which rows wait for their partner bodies' iterations and each
+ * contact's and joint's dual update is fused into the next iteration's primal row of the body
+ * that owns it;
  * AVBD_ITERATIONS_PER_COLOUR launches each colour and the dual sweep separately. Both give
  * the same bits. avbd_iteration_mode reports the mode the next step runs in (the
- * per-colour form where the device cannot hold the persistent launch, and while the
- * differentiable step records). */
+ * per-colour form where the device cannot hold the persistent launch). */
 int avbd_set_iteration_mode(AvbdContext *ctx, int32_t mode);
 int avbd_iteration_mode(AvbdContext *ctx, int32_t *mode);
 
@@ -487,14 +487,17 @@ int avbd_reset_profile(AvbdContext *ctx);
  *
  * Along the way it tapes every step's decisions and replays the frozen-branch map in double
  * precision, keeping a snapshot of that replay every checkpoint_every steps; the FP32 world
- * ends exactly where avbd_step(ctx, nsteps) would leave it.
+ * ends exactly where avbd_step(ctx, nsteps) would leave it. The replay of the last
+ * checkpoint segment also keeps its state at every iteration for the backward to start with,
+ * where that takes at most 1 GiB of device memory (above, the backward replays the segment);
+ * it stays allocated until the context goes, whether or not a backward follows.
  *
  * avbd_adjoint_backward takes the gradient of a loss with respect to the final state
  * (host arrays in list order: position n x 3, orientation n x 4 (x, y, z, w), velocity
  * n x 3, angular velocity n x 3; NULL = zero) and writes into the non-NULL host arrays of
  * AvbdAdjointGrad the gradient with respect to the state before the forward steps and the
- * parameters. Per checkpoint segment it replays the segment again, keeping the state at
- * every iteration, and sweeps it in reverse. It leaves the FP32 world untouched. The
+ * parameters. Per checkpoint segment it replays the segment again (but for a last one that the
+ * forward kept), keeping the state at every iteration, and sweeps it in reverse. It leaves the FP32 world untouched. The
  * forward must be the last thing that changed the world (a step, a body write or a load
  * in between is refused), and parameters and colouring mode must be the same.
  *
