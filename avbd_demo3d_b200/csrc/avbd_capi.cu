@@ -1111,9 +1111,10 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
         CHECK(reserve(ctx, ctx->bpKeysAlt, n, false));
         CHECK(reserve(ctx, ctx->sapVals, n, false));
         CHECK(reserve(ctx, ctx->sapValsAlt, n, false));
-        const int sweepBlocks = grid_for(n, SAP_WARPS);
-        CHECK(reserve(ctx, ctx->pairCount, n, false));
-        CHECK(reserve(ctx, ctx->pairOffset, n, false));
+        const int parts = sap_parts(n), items = n * parts, sweepBlock = sap_block(n, parts);
+        const int sweepBlocks = grid_for(items, sweepBlock / 32);
+        CHECK(reserve(ctx, ctx->pairCount, items, false));
+        CHECK(reserve(ctx, ctx->pairOffset, items, false));
         k_sap_axis<<<W, SAP_TILE, 0, ctx->stream>>>(B, ctx->worldStart.p, ctx->sapAxis.p);
         LAUNCHED();
         k_sap_keys<<<grid_for(n, 256), 256, 0, ctx->stream>>>(B, ctx->bodyWorld.p, ctx->sapAxis.p, ctx->bpKeys.p,
@@ -1130,24 +1131,24 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
         CU(cub::DeviceRadixSort::SortPairs(ctx->cubTemp.p, bytes, dk, dv, n, 0, endBit, ctx->stream));
         ctx->launches++;
         DevForces F = dev_forces(ctx);
-        k_sap_sweep<false><<<sweepBlocks, SAP_BLOCK, 0, ctx->stream>>>(
+        k_sap_sweep<false><<<sweepBlocks, sweepBlock, 0, ctx->stream>>>(
             B, F, ctx->sapAxis.p, ctx->worldStart.p, dk.Current(), dv.Current(), n, ctx->pairCount.p, nullptr, 0, 0,
-            cnt);
+            parts, cnt);
         LAUNCHED();
-        CHECK(scan_counts(ctx, ctx->pairCount.p, ctx->pairOffset.p, n, 0));
+        CHECK(scan_counts(ctx, ctx->pairCount.p, ctx->pairOffset.p, items, 0));
         ctx->launches++;
         if (deviceCounts)
         {
-            k_bp_commit<<<1, 1, 0, ctx->stream>>>(ctx->stepState.p, ctx->pairOffset.p, ctx->pairCount.p, n, nullptr,
+            k_bp_commit<<<1, 1, 0, ctx->stream>>>(ctx->stepState.p, ctx->pairOffset.p, ctx->pairCount.p, items, nullptr,
                                                   nullptr, 0, nullptr, cnt, (long long)man_capacity(ctx));
             LAUNCHED();
-            k_sap_sweep<true><<<sweepBlocks, SAP_BLOCK, 0, ctx->stream>>>(
+            k_sap_sweep<true><<<sweepBlocks, sweepBlock, 0, ctx->stream>>>(
                 B, dev_forces(ctx), ctx->sapAxis.p, ctx->worldStart.p, dk.Current(), dv.Current(), n, ctx->pairCount.p,
-                ctx->pairOffset.p, 0, 0, cnt, ctx->stepState.p);
+                ctx->pairOffset.p, 0, 0, parts, cnt, ctx->stepState.p);
             LAUNCHED();
             return AVBD_OK;
         }
-        k_total<<<1, 1, 0, ctx->stream>>>(ctx->pairOffset.p, ctx->pairCount.p, n, ctx->hScalars);
+        k_total<<<1, 1, 0, ctx->stream>>>(ctx->pairOffset.p, ctx->pairCount.p, items, ctx->hScalars);
         LAUNCHED();
         CU(cudaStreamSynchronize(ctx->stream));
         CHECK(nonfinite_checked(ctx));
@@ -1156,9 +1157,9 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
         {
             CHECK(reserve_manifolds(ctx, ctx->man[ctx->cur], (size_t)(M0 + P1), (size_t)M0));
             DevForces F2 = dev_forces(ctx);
-            k_sap_sweep<true><<<sweepBlocks, SAP_BLOCK, 0, ctx->stream>>>(
+            k_sap_sweep<true><<<sweepBlocks, sweepBlock, 0, ctx->stream>>>(
                 B, F2, ctx->sapAxis.p, ctx->worldStart.p, dk.Current(), dv.Current(), n, ctx->pairCount.p,
-                ctx->pairOffset.p, M0, (unsigned long long)ctx->nextSeq, cnt);
+                ctx->pairOffset.p, M0, (unsigned long long)ctx->nextSeq, parts, cnt);
             LAUNCHED();
         }
     }

@@ -1751,16 +1751,32 @@ __global__ void k_sap_keys(DevBodies B, const int *bodyWorld, const int *axis, u
 //
 // An interval's candidates are one stretch of its world's sorted keys: minima ascend, so the
 // first that starts past the maximum ends it (looked for among the next 32, then by a 32-way
-// search). A warp takes an interval of up to SAP_ALONE candidates; a longer one is left to its
-// block's 32 warps together, since the ground's interval holds every body of its world and one
-// warp walking it would be the step. counts[i] keep the sweep's order through the scan.
+// search). `parts` warps share an interval, a contiguous part each: as many as the chip has for
+// n intervals (SAP_RESIDENT), because a hit walks a force list, and one warp walking that of the
+// ground's interval, which holds every body of its world, would be the step. Parts of more than
+// SAP_ALONE candidates are left to the block's 32 warps together. counts[parts i + part] keep the
+// sweep's order through the scan (the block's whole interval counts as part 0). The emission
+// passes over parts without new pairs.
 // Bound by the latency of a warp's loads in one world, by issue in large batches. A step by a
 // thread an interval / by 32 warps an interval / so (us): 4,096 worlds of 7 bodies 730 / 1,085 /
-// 665, of 37 bodies 2,390 / 4,710 / 2,330; 64 uneven worlds 4,950 / 1,553 / 1,015; one world of
-// 1,860 bodies 3,040 / 267 / 254, of 20,737 30,460 / 997 / 787. SAP_ALONE at 128 / 512 / 2,048:
-// 1,860 bodies 282 / 255 / 361, 512 worlds 1,943 / 1,882 / 2,041, 65,537 bodies 2,088 / 2,050 /
-// 1,864 a step.
+// 680, of 37 bodies 2,390 / 4,710 / 2,370; 64 uneven worlds 4,950 / 1,553 / 1,034; one world of
+// 1,860 bodies 3,040 / 273 / 259, of 20,737 30,460 / 1,004 / 804; of 491 bodies 231 by 32 warps,
+// 227 so. Twice the warps (SAP_RESIDENT): 1,860 bodies 276, 181 bodies 200 for 196. SAP_ALONE at
+// 128 / 512 / 2,048, one warp an interval: 1,860 bodies 282 / 255 / 361, 512 worlds 1,943 / 1,882 /
+// 2,041, 65,537 bodies 2,088 / 2,050 / 1,864.
 constexpr int SAP_BLOCK = 1024, SAP_WARPS = SAP_BLOCK / 32, SAP_ALONE = 512, SAP_AHEAD = 4;
+constexpr int SAP_RESIDENT = 148 * SAP_WARPS; // warps the chip keeps of the sweep (64 registers a thread)
+constexpr int SAP_SMALL_BLOCK = 256;
+// Warps to an interval of n, and the block that goes with them: 32 warps where a part can be too
+// long for one.
+inline int sap_parts(int n)
+{
+    int parts = 1;
+    while (parts < SAP_WARPS && 2ll * parts * n <= SAP_RESIDENT)
+        parts *= 2;
+    return parts;
+}
+inline int sap_block(int n, int parts) { return n > SAP_ALONE * parts ? SAP_BLOCK : SAP_SMALL_BLOCK; }
 static_assert(SAP_WARPS == 32, "a warp's lanes stand for the block's warps");
 
 AVBD_DEV int sap_end(const unsigned long long *keys, int first, int last, unsigned long long top, int lane)
@@ -1798,8 +1814,8 @@ template <bool EMIT>
 __global__ void __launch_bounds__(SAP_BLOCK) k_sap_sweep(DevBodies B, DevForces F, const int *axis,
                                                          const int *worldStart, const unsigned long long *keys,
                                                          const int *vals, int n, int *counts, const int *offsets,
-                                                         int base, unsigned long long seqBase, StepCounters *cnt,
-                                                         const StepState *st = nullptr)
+                                                         int base, unsigned long long seqBase, int parts,
+                                                         StepCounters *cnt, const StepState *st = nullptr)
 {
     constexpr unsigned ALL = 0xFFFFFFFFu;
     if (EMIT && st)
@@ -1811,7 +1827,8 @@ __global__ void __launch_bounds__(SAP_BLOCK) k_sap_sweep(DevBodies B, DevForces 
     }
     __shared__ int longEnd[SAP_WARPS], longFound[SAP_WARPS], tileFound[2][SAP_WARPS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int i0 = (int)blockIdx.x * SAP_WARPS, i = i0 + warp;
+    const long long item0 = (long long)blockIdx.x * (blockDim.x >> 5), item = item0 + warp;
+    const int i = (int)(item / parts), part = (int)(item % parts);
     const unsigned lower = (1u << lane) - 1u;
     PairTally tally;
     auto emit = [&](int m, int a, int b) {
@@ -1820,7 +1837,7 @@ __global__ void __launch_bounds__(SAP_BLOCK) k_sap_sweep(DevBodies B, DevForces 
         F.man.n[m] = 0;
     };
     int forBlock = 0;
-    if (i < n && (!EMIT || counts[i] > 0)) // warp-uniform
+    if (i < n && (!EMIT || counts[item] > 0)) // warp-uniform
     {
         const int world = (int)(keys[i] >> 32), a = vals[i];
         const float3 pa = xyz(B.pos[a]);
@@ -1829,24 +1846,31 @@ __global__ void __launch_bounds__(SAP_BLOCK) k_sap_sweep(DevBodies B, DevForces 
         const float ahi = comp(pa, axis[world]) + ra + 0.0f;
         const unsigned long long top = ((unsigned long long)world << 32) | float_order(ahi);
         const int end = sap_end(keys, i + 1, worldStart[world + 1], top, lane);
-        if (!EMIT && lane == 0)
+        if (!EMIT && lane == 0 && part == 0)
             tally.checks += (unsigned)(end - (i + 1));
-        if (end - (i + 1) > SAP_ALONE)
-            forBlock = end;
+        const int len = end - (i + 1);
+        if (len > SAP_ALONE * parts)
+        {
+            forBlock = part == 0 ? end : 0;
+            if (!EMIT && part > 0 && lane == 0)
+                counts[item] = 0;
+        }
         else
         {
+            const int chunk = (len + 32 * parts - 1) / (32 * parts) * 32;
+            const int first = i + 1 + part * chunk, last = min(first + chunk, end);
             int found = 0;
-            const int out = EMIT ? base + offsets[i] : 0;
-            for (int at = i + 1; at < end; at += 32 * SAP_AHEAD)
+            const int out = EMIT ? base + offsets[item] : 0;
+            for (int at = first; at < last; at += 32 * SAP_AHEAD)
             {
-                const int rounds = (end - at + 31) / 32; // of the SAP_AHEAD, those that hold a candidate
+                const int rounds = (last - at + 31) / 32; // of the SAP_AHEAD, those that hold a candidate
                 int b[SAP_AHEAD];
                 float4 pb[SAP_AHEAD];
                 float rb[SAP_AHEAD];
 #pragma unroll
                 for (int u = 0; u < SAP_AHEAD; ++u)
                     if (u < rounds)
-                        b[u] = vals[min(at + 32 * u + lane, end - 1)];
+                        b[u] = vals[min(at + 32 * u + lane, last - 1)];
 #pragma unroll
                 for (int u = 0; u < SAP_AHEAD; ++u)
                     if (u < rounds)
@@ -1860,7 +1884,7 @@ __global__ void __launch_bounds__(SAP_BLOCK) k_sap_sweep(DevBodies B, DevForces 
                     if (u >= rounds)
                         break;
                     const bool fresh =
-                        at + 32 * u + lane < end && sap_test(F, a, pa, ra, b[u], xyz(pb[u]), rb[u], tally);
+                        at + 32 * u + lane < last && sap_test(F, a, pa, ra, b[u], xyz(pb[u]), rb[u], tally);
                     const unsigned mask = __ballot_sync(ALL, fresh);
                     if (EMIT && fresh)
                         emit(out + found + __popc(mask & lower), a, b[u]);
@@ -1868,8 +1892,14 @@ __global__ void __launch_bounds__(SAP_BLOCK) k_sap_sweep(DevBodies B, DevForces 
                 }
             }
             if (!EMIT && lane == 0)
-                counts[i] = found;
+                counts[item] = found;
         }
+    }
+    if (blockDim.x < SAP_BLOCK) // no part can be too long (sap_block)
+    {
+        if (!EMIT)
+            block_tally(cnt, tally);
+        return;
     }
     if (lane == 0)
     {
@@ -1880,12 +1910,12 @@ __global__ void __launch_bounds__(SAP_BLOCK) k_sap_sweep(DevBodies B, DevForces 
     int tile = 0;
     for (unsigned longs = __ballot_sync(ALL, longEnd[lane] != 0); longs; longs &= longs - 1)
     {
-        const int w = __ffs((int)longs) - 1, end = longEnd[w];
-        const int a = vals[i0 + w];
+        const int w = __ffs((int)longs) - 1, end = longEnd[w], iw = (int)((item0 + w) / parts);
+        const int a = vals[iw];
         const float3 pa = xyz(B.pos[a]);
         const float ra = B.sizeRad[a].w;
-        int out = EMIT ? base + offsets[i0 + w] : 0;
-        for (int at = i0 + w + 1; at < end; at += SAP_BLOCK)
+        int out = EMIT ? base + offsets[item0 + w] : 0;
+        for (int at = iw + 1; at < end; at += SAP_BLOCK)
         {
             const int j = at + (int)threadIdx.x;
             bool fresh = false;
@@ -1917,7 +1947,7 @@ __global__ void __launch_bounds__(SAP_BLOCK) k_sap_sweep(DevBodies B, DevForces 
     {
         __syncthreads();
         if (lane == 0 && forBlock != 0)
-            counts[i] = longFound[warp];
+            counts[item] = longFound[warp];
         block_tally(cnt, tally);
     }
 }

@@ -1,6 +1,7 @@
 """The sweep-and-prune sweep where its split turns: intervals at the most candidates a warp takes
-alone, at the block's tiles, several long ones in one block, and batches that mix worlds of a few
-bodies with a large one; pairs, order and counters against the CPU oracle."""
+alone, at the block's tiles, several long ones in one block, worlds at the sizes where an interval
+gets more or fewer warps, and batches that mix worlds of a few bodies with a large one; pairs,
+order and counters against the CPU oracle."""
 import numpy as np
 import pytest
 
@@ -62,6 +63,18 @@ def test_many_long_intervals_in_a_block(gpu, n):
         o.step(1)
         assert_same_state(g, o, f"{sc.name} step {s + 1}")
     g.close()
+
+
+@pytest.mark.parametrize("bodies", [148, 149, 296, 297, 592, 593, 1184, 1185, 2368, 2369, 4737])
+def test_warps_to_an_interval(gpu, bodies):
+    for sc in (row(bodies - 1), scenes.stack_grid(1, (bodies - 1) // 8, 8, seed=2, params=sap())):
+        o = checkers.World(sc, "oracle", order_mode=1)
+        g = same_pairs(sc, [o])
+        for s in range(2):
+            g.step(1)
+            o.step(1)
+            assert_same_state(g, o, f"{sc.name} step {s + 1}")
+        g.close()
 
 
 def test_small_worlds_beside_a_large_one(gpu):
