@@ -439,7 +439,8 @@ bool wide_possible(const AvbdContext *ctx) { return ctx->wideBlocks > 0 && ctx->
 // same bits, so an old count costs time alone.
 bool choose_wide(const AvbdContext *ctx)
 {
-    if (!wide_possible(ctx))
+    // a negative penalty has no place in the wide kernel's words: its sign bit is their version's
+    if (!wide_possible(ctx) || ctx->params.betaLin < 0.0f)
         return false;
     const int colours = ctx->pendingFast > 0 ? *(volatile const int *)&ctx->hState->nColours : ctx->nColours;
     const int solved = ((volatile const int *)ctx->hColourStarts)[1];

@@ -38,10 +38,10 @@
 // does.
 //
 // contactFlow, two words per slot: (pen.xyz, C0.z) with the low bit of the version in the sign
-// of pen.x (a penalty is at least PENALTY_MIN; a reader is at most one version behind), and
-// (lambda.xyz, version << 1 | stick). jointFlow, four words per joint: (penLin, version << 1 |
-// broken) (penAng, version) (lamLin, version) (lamAng, version). The contact and joint records
-// themselves are written once, with the last update.
+// of pen.x (a penalty is at least PENALTY_MIN and its ramp not negative, choose_wide; a reader is
+// at most one version behind), and (lambda.xyz, version << 1 | stick). jointFlow, four words per
+// joint: (penLin, version << 1 | broken) (penAng, version) (lamLin, version) (lamAng, version).
+// The contact and joint records themselves are written once, with the last update.
 #pragma once
 
 namespace avbd
