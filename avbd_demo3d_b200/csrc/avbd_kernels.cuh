@@ -1015,8 +1015,8 @@ AVBD_DEV void bp_pairs(long long tid, const DevBodies &B, const DevForces &F, co
         };
         // The entries from j on that belong to a run, four keys and spheres in flight. An emission
         // searches only where a lane found more than it could record: one at a time there, or the
-        // four set the registers of all its lanes (52, and 32 so: the broadphase alone of 4,096
-        // worlds, which emits every pair, 2.63 -> 2.53 ms).
+        // four set the registers of all its lanes (52, and 32 or 42 so: the broadphase alone of
+        // 4,096 worlds, which emits every pair, 2.63 -> 2.53 ms).
         constexpr int AHEAD = EMIT ? 1 : 4;
         auto search = [&](int j, unsigned long long run) {
             for (;; j += AHEAD)
@@ -1598,7 +1598,7 @@ __global__ void k_bp_large_large(DevForces F, const int *large, const float4 *la
 
 // A device step's emission: the grid entries' new pairs, and after their blocks the large
 // bodies'.
-__global__ void __launch_bounds__(128, 16)
+__global__ void __launch_bounds__(128, 12) // 42 registers: at 32 spills cost 65,536 boxes 0.3 % of a step
     k_bp_emit(DevBodies B, DevForces F, DevGrid G, const unsigned long long *keys, const float4 *spheres, int nBinned,
               HashTable cells, const int *large, const float4 *largeLo, const float4 *largeHi,
               const unsigned long long *largeKeys, int largeTotal, HashTable largeCells, float dt, int *counts,
