@@ -1767,6 +1767,7 @@ __global__ void k_sap_keys(DevBodies B, const int *bodyWorld, const int *axis, u
 constexpr int SAP_BLOCK = 1024, SAP_WARPS = SAP_BLOCK / 32, SAP_ALONE = 512, SAP_AHEAD = 4;
 constexpr int SAP_RESIDENT = 148 * SAP_WARPS; // warps the chip keeps of the sweep (64 registers a thread)
 constexpr int SAP_SMALL_BLOCK = 256;
+constexpr unsigned SAP_INF = 0xFF800000u; // float_order(infinity)
 // Warps to an interval of n, and the block that goes with them: 32 warps where a part can be too
 // long for one.
 inline int sap_parts(int n)
@@ -1779,12 +1780,19 @@ inline int sap_parts(int n)
 inline int sap_block(int n, int parts) { return n > SAP_ALONE * parts ? SAP_BLOCK : SAP_SMALL_BLOCK; }
 static_assert(SAP_WARPS == 32, "a warp's lanes stand for the block's warps");
 
+// The end of an interval's candidates, keys[first] .. keys[last - 1] being the later ones of its
+// world. Minima that are NaN end no walk: those sorted after infinity are all candidates once
+// reached (NaN of the other sign sort before everything).
 AVBD_DEV int sap_end(const unsigned long long *keys, int first, int last, unsigned long long top, int lane)
 {
     constexpr unsigned ALL = 0xFFFFFFFFu;
-    const int next = __popc(__ballot_sync(ALL, first + lane < last && keys[first + lane] <= top));
+    const unsigned long long own = first + lane < last ? keys[first + lane] : ~0ull;
+    const int next = __popc(__ballot_sync(ALL, first + lane < last && own <= top));
     if (next < 32)
-        return first + next;
+    {
+        const unsigned end = __shfl_sync(ALL, (unsigned)own, next);
+        return end > SAP_INF ? last : first + next;
+    }
     int lo = first + 32, hi = last; // keys[lo - 1] <= top < keys[hi]
     while (lo < hi)
     {
@@ -1794,7 +1802,7 @@ AVBD_DEV int sap_end(const unsigned long long *keys, int first, int last, unsign
         hi = min(hi, lo + below * step);
         lo = below > 0 ? lo + (below - 1) * step + 1 : hi;
     }
-    return hi;
+    return hi < last && (unsigned)keys[hi] > SAP_INF ? last : hi;
 }
 
 // Candidate b of body a: a new pair?
@@ -1844,7 +1852,8 @@ __global__ void __launch_bounds__(SAP_BLOCK) k_sap_sweep(DevBodies B, DevForces 
         const float ra = B.sizeRad[a].w;
         // the last key inside is at most (world, maximum); a maximum of -0 counts as +0, as in a comparison
         const float ahi = comp(pa, axis[world]) + ra + 0.0f;
-        const unsigned long long top = ((unsigned long long)world << 32) | float_order(ahi);
+        // (a maximum that is NaN ends at none)
+        const unsigned long long top = ((unsigned long long)world << 32) | (isnan(ahi) ? ~0u : float_order(ahi));
         const int end = sap_end(keys, i + 1, worldStart[world + 1], top, lane);
         if (!EMIT && lane == 0 && part == 0)
             tally.checks += (unsigned)(end - (i + 1));
