@@ -1112,7 +1112,7 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
         CHECK(reserve(ctx, ctx->bpKeysAlt, n, false));
         CHECK(reserve(ctx, ctx->sapVals, n, false));
         CHECK(reserve(ctx, ctx->sapValsAlt, n, false));
-        const int parts = sap_parts(n), items = n * parts, sweepBlock = sap_block(n, parts);
+        const int partsLog = sap_parts_log(n), items = n << partsLog, sweepBlock = sap_block(n, 1 << partsLog);
         const int sweepBlocks = grid_for(items, sweepBlock / 32);
         CHECK(reserve(ctx, ctx->pairCount, items, false));
         CHECK(reserve(ctx, ctx->pairOffset, items, false));
@@ -1134,7 +1134,7 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
         DevForces F = dev_forces(ctx);
         k_sap_sweep<false><<<sweepBlocks, sweepBlock, 0, ctx->stream>>>(
             B, F, ctx->sapAxis.p, ctx->worldStart.p, dk.Current(), dv.Current(), n, ctx->pairCount.p, nullptr, 0, 0,
-            parts, cnt);
+            partsLog, cnt);
         LAUNCHED();
         CHECK(scan_counts(ctx, ctx->pairCount.p, ctx->pairOffset.p, items, 0));
         ctx->launches++;
@@ -1145,7 +1145,7 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
             LAUNCHED();
             k_sap_sweep<true><<<sweepBlocks, sweepBlock, 0, ctx->stream>>>(
                 B, dev_forces(ctx), ctx->sapAxis.p, ctx->worldStart.p, dk.Current(), dv.Current(), n, ctx->pairCount.p,
-                ctx->pairOffset.p, 0, 0, parts, cnt, ctx->stepState.p);
+                ctx->pairOffset.p, 0, 0, partsLog, cnt, ctx->stepState.p);
             LAUNCHED();
             return AVBD_OK;
         }
@@ -1160,7 +1160,7 @@ int broadphase(AvbdContext *ctx, bool deviceCounts = false)
             DevForces F2 = dev_forces(ctx);
             k_sap_sweep<true><<<sweepBlocks, sweepBlock, 0, ctx->stream>>>(
                 B, F2, ctx->sapAxis.p, ctx->worldStart.p, dk.Current(), dv.Current(), n, ctx->pairCount.p,
-                ctx->pairOffset.p, M0, (unsigned long long)ctx->nextSeq, parts, cnt);
+                ctx->pairOffset.p, M0, (unsigned long long)ctx->nextSeq, partsLog, cnt);
             LAUNCHED();
         }
     }

@@ -1759,9 +1759,9 @@ __global__ void k_sap_keys(DevBodies B, const int *bodyWorld, const int *axis, u
 // passes over parts without new pairs.
 // Bound by the latency of a warp's loads in one world, by issue in large batches. A step by a
 // thread an interval / by 32 warps an interval / so (us): 4,096 worlds of 7 bodies 730 / 1,085 /
-// 680, of 37 bodies 2,390 / 4,710 / 2,370; 64 uneven worlds 4,950 / 1,553 / 1,034; one world of
-// 1,860 bodies 3,040 / 273 / 259, of 20,737 30,460 / 1,004 / 804; of 491 bodies 231 by 32 warps,
-// 227 so. Twice the warps (SAP_RESIDENT): 1,860 bodies 276, 181 bodies 200 for 196. SAP_ALONE at
+// 663, of 37 bodies 2,390 / 4,705 / 2,320; 64 uneven worlds 4,950 / 1,547 / 1,006; one world of
+// 1,860 bodies 3,040 / 264 / 245, of 20,737 30,460 / 996 / 785; of 491 bodies 226 by 32 warps,
+// 224 so. Twice the warps (SAP_RESIDENT): 1,860 bodies 276, 181 bodies 200 for 196. SAP_ALONE at
 // 128 / 512 / 2,048, one warp an interval: 1,860 bodies 282 / 255 / 361, 512 worlds 1,943 / 1,882 /
 // 2,041, 65,537 bodies 2,088 / 2,050 / 1,864.
 constexpr int SAP_BLOCK = 1024, SAP_WARPS = SAP_BLOCK / 32, SAP_ALONE = 512, SAP_AHEAD = 4;
@@ -1770,28 +1770,29 @@ constexpr int SAP_SMALL_BLOCK = 256;
 constexpr unsigned SAP_INF = 0xFF800000u; // float_order(infinity)
 // Warps to an interval of n, and the block that goes with them: 32 warps where a part can be too
 // long for one.
-inline int sap_parts(int n)
+inline int sap_parts_log(int n)
 {
-    int parts = 1;
-    while (parts < SAP_WARPS && 2ll * parts * n <= SAP_RESIDENT)
-        parts *= 2;
-    return parts;
+    int log = 0;
+    while (1 << log < SAP_WARPS && (2ll << log) * n <= SAP_RESIDENT)
+        ++log;
+    return log;
 }
 inline int sap_block(int n, int parts) { return n > SAP_ALONE * parts ? SAP_BLOCK : SAP_SMALL_BLOCK; }
 static_assert(SAP_WARPS == 32, "a warp's lanes stand for the block's warps");
 
 // The end of an interval's candidates, keys[first] .. keys[last - 1] being the later ones of its
-// world. Minima that are NaN end no walk: those sorted after infinity are all candidates once
+// world (keys of the next world, up to n, are beyond any `top` of this one, so the first look does
+// not wait for `last`). Minima that are NaN end no walk: those sorted after infinity are all candidates once
 // reached (NaN of the other sign sort before everything).
-AVBD_DEV int sap_end(const unsigned long long *keys, int first, int last, unsigned long long top, int lane)
+AVBD_DEV int sap_end(const unsigned long long *keys, int first, int last, int n, unsigned long long top, int lane)
 {
     constexpr unsigned ALL = 0xFFFFFFFFu;
-    const unsigned long long own = first + lane < last ? keys[first + lane] : ~0ull;
-    const int next = __popc(__ballot_sync(ALL, first + lane < last && own <= top));
+    const unsigned long long own = first + lane < n ? keys[first + lane] : ~0ull;
+    const int next = __popc(__ballot_sync(ALL, own <= top));
     if (next < 32)
     {
         const unsigned end = __shfl_sync(ALL, (unsigned)own, next);
-        return end > SAP_INF ? last : first + next;
+        return first + next < last && end > SAP_INF ? last : first + next;
     }
     int lo = first + 32, hi = last; // keys[lo - 1] <= top < keys[hi]
     while (lo < hi)
@@ -1822,7 +1823,7 @@ template <bool EMIT>
 __global__ void __launch_bounds__(SAP_BLOCK) k_sap_sweep(DevBodies B, DevForces F, const int *axis,
                                                          const int *worldStart, const unsigned long long *keys,
                                                          const int *vals, int n, int *counts, const int *offsets,
-                                                         int base, unsigned long long seqBase, int parts,
+                                                         int base, unsigned long long seqBase, int partsLog,
                                                          StepCounters *cnt, const StepState *st = nullptr)
 {
     constexpr unsigned ALL = 0xFFFFFFFFu;
@@ -1836,7 +1837,7 @@ __global__ void __launch_bounds__(SAP_BLOCK) k_sap_sweep(DevBodies B, DevForces 
     __shared__ int longEnd[SAP_WARPS], longFound[SAP_WARPS], tileFound[2][SAP_WARPS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long long item0 = (long long)blockIdx.x * (blockDim.x >> 5), item = item0 + warp;
-    const int i = (int)(item / parts), part = (int)(item % parts);
+    const int parts = 1 << partsLog, i = (int)(item >> partsLog), part = (int)item & (parts - 1);
     const unsigned lower = (1u << lane) - 1u;
     PairTally tally;
     auto emit = [&](int m, int a, int b) {
@@ -1845,16 +1846,17 @@ __global__ void __launch_bounds__(SAP_BLOCK) k_sap_sweep(DevBodies B, DevForces 
         F.man.n[m] = 0;
     };
     int forBlock = 0;
+    const unsigned long long key = i < n ? keys[i] : 0ull; // beside the count
     if (i < n && (!EMIT || counts[item] > 0)) // warp-uniform
     {
-        const int world = (int)(keys[i] >> 32), a = vals[i];
+        const int world = (int)(key >> 32), a = vals[i];
         const float3 pa = xyz(B.pos[a]);
         const float ra = B.sizeRad[a].w;
         // the last key inside is at most (world, maximum); a maximum of -0 counts as +0, as in a comparison
         const float ahi = comp(pa, axis[world]) + ra + 0.0f;
         // (a maximum that is NaN ends at none)
         const unsigned long long top = ((unsigned long long)world << 32) | (isnan(ahi) ? ~0u : float_order(ahi));
-        const int end = sap_end(keys, i + 1, worldStart[world + 1], top, lane);
+        const int end = sap_end(keys, i + 1, worldStart[world + 1], n, top, lane);
         if (!EMIT && lane == 0 && part == 0)
             tally.checks += (unsigned)(end - (i + 1));
         const int len = end - (i + 1);
@@ -1866,7 +1868,7 @@ __global__ void __launch_bounds__(SAP_BLOCK) k_sap_sweep(DevBodies B, DevForces 
         }
         else
         {
-            const int chunk = (len + 32 * parts - 1) / (32 * parts) * 32;
+            const int chunk = (len + 32 * parts - 1) >> (5 + partsLog) << 5;
             const int first = i + 1 + part * chunk, last = min(first + chunk, end);
             int found = 0;
             const int out = EMIT ? base + offsets[item] : 0;
@@ -1919,7 +1921,7 @@ __global__ void __launch_bounds__(SAP_BLOCK) k_sap_sweep(DevBodies B, DevForces 
     int tile = 0;
     for (unsigned longs = __ballot_sync(ALL, longEnd[lane] != 0); longs; longs &= longs - 1)
     {
-        const int w = __ffs((int)longs) - 1, end = longEnd[w], iw = (int)((item0 + w) / parts);
+        const int w = __ffs((int)longs) - 1, end = longEnd[w], iw = (int)((item0 + w) >> partsLog);
         const int a = vals[iw];
         const float3 pa = xyz(B.pos[a]);
         const float ra = B.sizeRad[a].w;
