@@ -56,10 +56,10 @@ def measured_peak():
 # (kernel_sources_sha, comments left out): when the code has changed since, the figure no
 # longer describes the kernel and the line reports no traffic.
 NCU_TRAFFIC = {
-    "k_iterations": {"bytes_per_launch": 30868224, "summary": "profiles/iterations_stacks65k_ncu.txt",
-                     "captured": "2026-12-04", "commit": "9466f58", "sources_sha": "6b8145f7b8c71b4a"},
-    "k_iterations_batched": {"bytes_per_launch": 9873686000, "summary": "profiles/iterations_batched4096_ncu.txt",
-                             "captured": "2026-12-04", "commit": "64ded38", "sources_sha": "6b8145f7b8c71b4a"},
+    "k_iterations": {"bytes_per_launch": 32673792, "summary": "profiles/iterations_stacks65k_ncu.txt",
+                     "captured": "2026-12-05", "commit": "dd2b8c8", "sources_sha": "cec47ceeef0cbde4"},
+    "k_iterations_batched": {"bytes_per_launch": 9872094976, "summary": "profiles/iterations_batched4096_ncu.txt",
+                             "captured": "2026-12-05", "commit": "dd2b8c8", "sources_sha": "cec47ceeef0cbde4"},
     "k_primal": {"bytes_per_launch": None, "summary": "profiles/primal_stacks65k_ncu.txt",
                  "captured": "2026-12-04", "sources_sha": ""},
 }
